@@ -25,10 +25,11 @@
 //                 cut by a chunk edge leaves partial sums.  Equal chunks keep
 //                 every thread busy whatever the scalar distribution.
 //  5. fixup       the chunk where a cut bucket starts sums its partials.
-//  6. reduce      per window, sum_b (b+1) B_b: running sums over groups of 16
-//                 buckets (one thread per group), then the weighted group sums
-//                 sum_g g R_g by bit planes (plain tree sums), one block each.
-//  7. finish      one thread per window folds the planes into the window sum.
+//  6. reduce      per window, sum_b (b+1) B_b by a tree over its buckets whose
+//                 nodes carry their sum and the sums over every bit plane of
+//                 the index, four lanes per addition; where buckets fill the
+//                 GPU, running sums over groups of buckets come first.
+//  7. finish      one block per window shifts the planes and adds them up.
 //  8. host        sum_w 2^(c w) S_w (c doublings between windows) and the
 //                 affine normalisation on the host: a few hundred group
 //                 operations that one GPU thread would take ~1 ms for.
@@ -44,6 +45,7 @@
 #include <vector>
 
 #include "ec.cuh"
+#include "ec_quad.cuh"
 #include "host_ec.hpp"
 #include "runtime.hpp"
 
@@ -51,7 +53,6 @@ namespace mzk {
 
 namespace {
 
-constexpr int kGroupLog = 6;       // log2 of the buckets per running-sum group (fewer when nb is smaller)
 constexpr int kAccThreads = 128;   // threads per block of the accumulate kernel
 constexpr int kReduceThreads = 128;
 constexpr uint32_t kNoKey = 0xffffffffu;
@@ -61,33 +62,15 @@ struct MsmShape {
     int windows;    // number of windows
     uint32_t nb;    // buckets per window = 2^(c-1)
     uint32_t keys;  // windows * nb
-    int glen_log;   // log2 of the buckets per running-sum group
-    uint32_t groups;  // running-sum groups per window = nb >> glen_log
-    int planes;     // log2(groups)
 };
 
-// glen_log: log2 of the buckets per running-sum group, at most c - 1
-MsmShape make_shape(int c, int glen_log = kGroupLog) {
+MsmShape make_shape(int c) {
     MsmShape s;
     s.c = c;
     s.windows = (256 + c - 1) / c;
     s.nb = 1u << (c - 1);
     s.keys = s.nb * (uint32_t)s.windows;
-    s.glen_log = c - 1 < glen_log ? c - 1 : glen_log;
-    s.groups = s.nb >> s.glen_log;
-    s.planes = 0;
-    while ((1u << s.planes) < s.groups) s.planes++;
     return s;
-}
-
-// Running-sum group length for a call whose windows hold `keys` buckets in
-// all: long groups (fewer plane sums) while there are still >= 32768 groups
-// to fill the GPU, shorter ones for small MSMs, whose group chains would
-// otherwise be latency-bound (a group is one thread's chain of 2L additions).
-int group_log_for(uint64_t keys) {
-    int g = 2;
-    while (g < kGroupLog && (keys >> (g + 1)) >= 32768) g++;
-    return g;
 }
 
 __device__ __forceinline__ uint32_t fr_limb(const Fr& s, int i) {
@@ -412,85 +395,106 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
     flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, owner_key);
 }
 
-// A cut bucket is finished by the chunk where it starts.  Short spans are summed
-// by that thread; a bucket spanning many chunks (a heavy bucket: scalars 0/1,
-// a nearly empty top window) is queued for k_fixup_long.
-constexpr uint32_t kShortSpan = 32;
+// A cut bucket is finished by the chunk where it starts: one quad of lanes per
+// chunk, since the additions of a span are a serial chain.  A bucket spanning
+// many chunks (a heavy bucket: scalars 0/1, a nearly empty top window) is
+// queued for k_fixup_long, whose 64 quads take ~30 us for any span up to 65: the
+// chain of 12 additions that a quad still takes itself costs ~55.  Device time
+// of both kernels, quads against lanes: proof of 2^14 rows (6 calls) 2.51 ->
+// 1.70 ms, 2^16 points 150 -> 70 us.
+constexpr uint32_t kShortSpan = 12;
 
-__global__ void k_fixup(const uint32_t* __restrict__ offsets, uint32_t keys, const Xyzz* __restrict__ partials,
-                        const int* __restrict__ owner_key, Xyzz* __restrict__ buckets, uint32_t* __restrict__ long_count,
-                        uint2* __restrict__ long_list) {
-    const uint32_t nthreads = gridDim.x * blockDim.x;  // same grid as k_accumulate
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = owner_key[t];
-    if (k < 0) return;
-    const uint32_t total = offsets[keys];
-    const uint32_t len = (total + nthreads - 1) / nthreads;
-    const uint32_t last = (offsets[k + 1] - 1) / len;
-    if (last - t > kShortSpan) {
-        const uint32_t slot = atomicAdd(long_count, 1u);
-        long_list[slot] = make_uint2(t, last);
-        return;
+// quads beyond `chunks` and chunks without an owner add nothing (whole warps
+// stay together in quad_add)
+__global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __restrict__ offsets, uint32_t keys,
+                                                          uint32_t chunks, const Xyzz* __restrict__ partials,
+                                                          const int* __restrict__ owner_key, Xyzz* __restrict__ buckets,
+                                                          uint32_t* __restrict__ long_count,
+                                                          uint2* __restrict__ long_list) {
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const int k = t < chunks ? owner_key[t] : -1;
+    uint32_t last = t;
+    Fp acc = fp_zero();
+    bool mine = k >= 0;
+    if (mine) {
+        const uint32_t total = offsets[keys];
+        const uint32_t len = (total + chunks - 1) / chunks;
+        last = (offsets[k + 1] - 1) / len;
+        if (last - t > kShortSpan) {
+            if ((threadIdx.x & 3) == 0) long_list[atomicAdd(long_count, 1u)] = make_uint2(t, last);
+            last = t;
+            mine = false;
+        } else {
+            acc = quad_load(&partials[2 * (size_t)t + 1]);
+        }
     }
-    Xyzz acc = load_xyzz(&partials[2 * (size_t)t + 1]);
-    for (uint32_t u = t + 1; u <= last; u++) acc = xyzz_add(acc, load_xyzz(&partials[2 * (size_t)u]));
-    store_xyzz(&buckets[k], acc);
+    for (uint32_t u = t + 1; __any_sync(0xffffffffu, u <= last); u++)
+        acc = quad_add(acc, u <= last ? quad_load(&partials[2 * (size_t)u]) : fp_zero());
+    if (mine) quad_store(&buckets[k], acc);
 }
 
-// one block per queued heavy bucket: strided partial sums, then a tree
-__global__ void __launch_bounds__(kReduceThreads) k_fixup_long(const int* __restrict__ owner_key,
-                                                               const Xyzz* __restrict__ partials,
-                                                               const uint32_t* __restrict__ long_count,
-                                                               const uint2* __restrict__ long_list,
-                                                               Xyzz* __restrict__ buckets) {
-    extern __shared__ uint4 smem_raw[];
-    Xyzz* sm = reinterpret_cast<Xyzz*>(smem_raw);
+// one block per queued heavy bucket: its quads sum strided shares of the span,
+// then the block's points are added pairwise
+constexpr int kLongThreads = 256;
+
+__global__ void __launch_bounds__(kLongThreads) k_fixup_long(const int* __restrict__ owner_key,
+                                                             const Xyzz* __restrict__ partials,
+                                                             const uint32_t* __restrict__ long_count,
+                                                             const uint2* __restrict__ long_list,
+                                                             Xyzz* __restrict__ buckets) {
+    constexpr uint32_t kQuads = kLongThreads / 4;
+    __shared__ Xyzz sm[kQuads];
+    const uint32_t quad = threadIdx.x >> 2;
     for (uint32_t item = blockIdx.x; item < *long_count; item += gridDim.x) {
         const uint2 tl = long_list[item];
         const uint32_t t = tl.x, last = tl.y;
-        Xyzz acc;
-        if (threadIdx.x == 0) acc = load_xyzz(&partials[2 * (size_t)t + 1]);
-        else xyzz_set_inf(acc);
-        for (uint32_t u = t + 1 + threadIdx.x; u <= last; u += blockDim.x)
-            acc = xyzz_add(acc, load_xyzz(&partials[2 * (size_t)u]));
-        sm[threadIdx.x] = acc;
+        Fp acc = quad == 0 ? quad_load(&partials[2 * (size_t)t + 1]) : fp_zero();
+        for (uint32_t u = t + 1 + quad; __any_sync(0xffffffffu, u <= last); u += kQuads)
+            acc = quad_add(acc, u <= last ? quad_load(&partials[2 * (size_t)u]) : fp_zero());
+        quad_store(&sm[quad], acc);
         __syncthreads();
-        for (int off = blockDim.x >> 1; off > 0; off >>= 1) {
-            if ((int)threadIdx.x < off) sm[threadIdx.x] = xyzz_add(sm[threadIdx.x], sm[threadIdx.x + off]);
+        for (uint32_t off = kQuads / 2; off > 0; off >>= 1) {
+            if ((quad & ~7u) < off) {  // warps stay together
+                const Fp r = quad_add(quad_load(&sm[quad]), quad < off ? quad_load(&sm[quad + off]) : fp_zero());
+                if (quad < off) quad_store(&sm[quad], r);
+            }
             __syncthreads();
         }
-        if (threadIdx.x == 0) store_xyzz(&buckets[owner_key[t]], sm[0]);
+        if (quad == 0) quad_store(&buckets[owner_key[t]], quad_load(&sm[0]));
         __syncthreads();
     }
 }
 
 // ---- bucket reduction over a table of windows ----
 //
-// A window's sum S = sum_{b=1}^{nb} b * B_b is reduced in three steps:
-//   1. running sums over groups of L = 2^glen_log consecutive buckets, top
-//      first: R_g = sum of the group's buckets, T_g = sum_i (i+1) B_{gL+i};
-//   2. plane sums: Q_j = sum of R_g over the groups g with bit j set, and
-//      T = sum_g T_g (each plane split over `split` blocks, then merged);
-//   3. S = T + L * sum_j 2^j Q_j (Horner, one thread per window).
-// One table row per window serves a single MSM and a batch of MSMs alike.
-struct WinDev {
+// A window's sum is S = sum_{b=1}^{nb} b B_b.  Its nb = 2^m buckets are merged
+// pairwise in a tree whose nodes hold the sum R of their leaves and, for every
+// bit t below the node's height, the plane sum P_t over the leaves whose index
+// has bit t set.  Merging two nodes adds R and every P_t of the halves and
+// gains the plane of its own height for free (the right half's R), so the
+// whole tree takes ~2 nb additions, as many as running sums, and is only m
+// additions deep.  Then S = R + sum_t 2^t P_t.
+//
+// k_tree runs 1..8 heights of it per launch, each block a subtree in shared
+// memory with one quad of lanes per addition (a quad addition takes a third of
+// the time of a one-lane addition, and these are chains).  Where a call has
+// buckets enough to fill the GPU with one-lane work anyway (kTreeKeys),
+// k_group_sums first folds groups of L = 2^glen buckets by running sums
+// (R_g = sum of the group's buckets, T_g = sum_i (i+1) B_{gL+i}, ~1/4 less
+// work per bucket than the quads) and the tree runs over the groups:
+// S = sum_g T_g + L sum_t 2^t P_t.  k_tree_finish shifts the planes of a window
+// side by side and adds them up.
+//
+// Bound by the latency of a product chain for few buckets and by the integer
+// multiply pipe for many.  Device time of the whole reduction, against running
+// sums over groups with one lane per addition, plane sums and a serial Horner
+// step per window: 4096 buckets (1000 points) 496 -> 94 us, 81920 (2^16
+// points) 1177 -> 265 us, 524288 (10^6 points) 1840 -> 1010 us.
+struct GroupWin {
     uint32_t key_start;    // first bucket key of the window
-    uint32_t nb;           // buckets in the window
     uint32_t group_start;  // first running-sum group of the window
-    uint32_t plane_start;  // first of its planes + 1 plane slots
     uint32_t glen_log;     // log2 of the buckets per group
-    int planes;            // log2 of the groups per window
 };
-
-__device__ __forceinline__ uint32_t find_win(const WinDev* wins, uint32_t n_wins, uint32_t v, bool by_plane) {
-    uint32_t lo = 0, hi = n_wins;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((by_plane ? wins[mid].plane_start : wins[mid].group_start) <= v) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
 
 // The bucket sets of an MSM over the same keys (one per part of a pipelined
 // MSM), added bucket by bucket; a key is empty in a set when its offsets
@@ -501,13 +505,19 @@ struct BucketSets {
     uint32_t n;
 };
 
+// group g leaves the pair T_g, R_g at out[2 g]
 __global__ void __launch_bounds__(kReduceThreads) k_group_sums(const BucketSets sets,
-                                                               const WinDev* __restrict__ wins, uint32_t n_wins,
-                                                               uint32_t total_groups, Xyzz* __restrict__ run_out,
-                                                               Xyzz* __restrict__ tot_out) {
+                                                               const GroupWin* __restrict__ wins, uint32_t n_wins,
+                                                               uint32_t total_groups, Xyzz* __restrict__ out) {
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= total_groups) return;
-    const WinDev wd = wins[find_win(wins, n_wins, gid, false)];
+    uint32_t lo = 0, hi = n_wins;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (wins[mid].group_start <= gid) lo = mid;
+        else hi = mid;
+    }
+    const GroupWin wd = wins[lo];
     const uint32_t key0 = wd.key_start + ((gid - wd.group_start) << wd.glen_log);
     Xyzz run, tot;
     xyzz_set_inf(run);
@@ -520,110 +530,235 @@ __global__ void __launch_bounds__(kReduceThreads) k_group_sums(const BucketSets 
                 run = xyzz_add(run, load_xyzz(&sets.buckets[s][key]));
         tot = xyzz_add(tot, run);
     }
-    store_xyzz(&run_out[gid], run);
-    store_xyzz(&tot_out[gid], tot);
+    store_xyzz(&out[2 * (size_t)gid], tot);
+    store_xyzz(&out[2 * (size_t)gid + 1], run);
 }
 
-// block b: plane slot b / split, part b % split of the window's groups.
-// Slot plane < planes sums R_g over the g with bit `plane` set; slot plane ==
-// planes sums T_g over all g.
-__global__ void __launch_bounds__(kReduceThreads) k_plane_sums(const Xyzz* __restrict__ run,
-                                                               const Xyzz* __restrict__ tot,
-                                                               const WinDev* __restrict__ wins, uint32_t n_wins,
-                                                               uint32_t split, Xyzz* __restrict__ partial) {
-    extern __shared__ uint4 smem_raw[];
-    Xyzz* sm = reinterpret_cast<Xyzz*>(smem_raw);
-    const uint32_t slot = blockIdx.x / split, part = blockIdx.x % split;
-    const WinDev wd = wins[find_win(wins, n_wins, slot, true)];
-    const int plane = (int)(slot - wd.plane_start);
-    const uint32_t groups = wd.nb >> wd.glen_log;
-    const uint32_t chunk = (groups + split - 1) / split;
-    const uint32_t g_end = min(groups, (part + 1) * chunk);
-    const Xyzz* src = (plane == wd.planes ? tot : run) + wd.group_start;
-    Xyzz acc;
-    xyzz_set_inf(acc);
-    for (uint32_t g = part * chunk + threadIdx.x; g < g_end; g += blockDim.x)
-        if (plane == wd.planes || ((g >> plane) & 1u)) acc = xyzz_add(acc, load_xyzz(&src[g]));
-    sm[threadIdx.x] = acc;
+// One launch of k_tree on one window: 2^b of its nodes per block.  A node has
+// v values: its planes (and T), R last; it leaves with v + b values.
+struct TreeWin {
+    uint32_t blk_start;  // the window's first block
+    uint32_t in_start;   // its first value (points)
+    uint32_t out_start;
+    uint32_t v, b;
+};
+constexpr uint32_t kTreePoints = 256;  // points of a block's subtree (48 KB of shared memory)
+
+// Values are merged in place.  Value j of the node over the leaves from L sits
+// in slot (L, j), its new plane t in the last slot of leaf L + 2^t (the R that
+// the right half left there), its R in the last slot of leaf L.
+// offsets (first launch over buckets only): key k is empty, and its bucket
+// never written, when offsets[k + 1] == offsets[k].
+__global__ void __launch_bounds__(256) k_tree(const Xyzz* __restrict__ in, const uint32_t* __restrict__ offsets,
+                                              const TreeWin* __restrict__ wins, uint32_t n_wins,
+                                              Xyzz* __restrict__ out) {
+    __shared__ Xyzz sm[kTreePoints];
+    uint32_t lo = 0, hi = n_wins;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (wins[mid].blk_start <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const TreeWin w = wins[lo];
+    const uint32_t blk = blockIdx.x - w.blk_start, v = w.v;
+    const uint32_t points = v << w.b, quads = blockDim.x >> 2, quad = threadIdx.x >> 2;
+    const uint32_t first = w.in_start + blk * points;
+    for (uint32_t i = quad; i < points; i += quads) {
+        const bool empty = offsets && offsets[first + i + 1] == offsets[first + i];
+        quad_store(&sm[i], empty ? fp_zero() : quad_load(&in[first + i]));
+    }
     __syncthreads();
-    for (int off = blockDim.x >> 1; off > 0; off >>= 1) {
-        if ((int)threadIdx.x < off) sm[threadIdx.x] = xyzz_add(sm[threadIdx.x], sm[threadIdx.x + off]);
+    for (uint32_t s = 0; s < w.b; s++) {
+        const uint32_t per = v + s, ops = per << (w.b - s - 1);
+        for (uint32_t o = quad; (o & ~7u) < ops; o += quads) {  // a warp's eight quads stay together
+            const uint32_t m = o / per, r = o % per;
+            const uint32_t left = m << (s + 1), half = 1u << s;
+            uint32_t dst = left * v + r;
+            if (r >= v) dst = (left + (1u << (r - v))) * v + v - 1;  // plane r - v gained below
+            const bool on = o < ops;
+            const uint32_t src = dst + half * v;
+            const Fp sum = quad_add(on ? quad_load(&sm[dst]) : fp_zero(), on ? quad_load(&sm[src]) : fp_zero());
+            // slot (left + half, v - 1), the R of the right half, is read here
+            // and stays: it is the merged node's plane s
+            if (on) quad_store(&sm[dst], sum);
+        }
         __syncthreads();
     }
-    if (threadIdx.x == 0) store_xyzz(&partial[blockIdx.x], sm[0]);
-}
-
-// q[slot] = sum of the slot's `split` partial plane sums
-__global__ void k_plane_merge(const Xyzz* __restrict__ partial, uint32_t slots, uint32_t split,
-                              Xyzz* __restrict__ q) {
-    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
-    if (slot >= slots) return;
-    Xyzz acc = load_xyzz(&partial[(size_t)slot * split]);
-    for (uint32_t p = 1; p < split; p++) acc = xyzz_add(acc, load_xyzz(&partial[(size_t)slot * split + p]));
-    store_xyzz(&q[slot], acc);
-}
-
-// S = T + L * sum_j 2^j Q_j, one thread per window
-__global__ void k_window_finish(const Xyzz* __restrict__ q_all, const WinDev* __restrict__ wins, uint32_t n_wins,
-                                Xyzz* __restrict__ out) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= n_wins) return;
-    const WinDev wd = wins[w];
-    const Xyzz* q = q_all + wd.plane_start;
-    Xyzz acc;
-    xyzz_set_inf(acc);
-    for (int j = wd.planes - 1; j >= 0; j--) {
-        acc = xyzz_dbl(acc);
-        acc = xyzz_add(acc, load_xyzz(&q[j]));
-    }
-    for (uint32_t b = 0; b < wd.glen_log; b++) acc = xyzz_dbl(acc);
-    acc = xyzz_add(acc, load_xyzz(&q[wd.planes]));
-    store_xyzz(&out[w], acc);
-}
-
-// the table rows of one MSM's windows, appended to `wins`
-void append_windows(const MsmShape& sh, uint64_t key_base, std::vector<WinDev>& wins, uint64_t& groups,
-                    uint64_t& slots) {
-    for (int w = 0; w < sh.windows; w++) {
-        WinDev wd;
-        wd.key_start = (uint32_t)(key_base + (uint64_t)w * sh.nb);
-        wd.nb = sh.nb;
-        wd.group_start = (uint32_t)groups;
-        wd.plane_start = (uint32_t)slots;
-        wd.glen_log = (uint32_t)sh.glen_log;
-        wd.planes = sh.planes;
-        wins.push_back(wd);
-        groups += sh.groups;
-        slots += (uint64_t)sh.planes + 1;
+    const uint32_t nv = v + w.b;
+    for (uint32_t i = quad; i < nv; i += quads) {
+        const uint32_t slot = i + 1 < v ? i : i + 1 == nv ? v - 1 : (1u << (i + 1 - v)) * v + v - 1;
+        quad_store(&out[w.out_start + blk * nv + i], quad_load(&sm[slot]));
     }
 }
 
-// blocks per plane slot: enough blocks to fill the GPU, at most one per
-// kReduceThreads groups of the largest window, at most 16
-uint32_t plane_split(uint64_t slots, uint32_t max_groups, int num_sms) {
-    const uint64_t want = ((uint64_t)num_sms * 8 + slots - 1) / slots;
-    const uint64_t cap = std::max<uint64_t>(1, max_groups / kReduceThreads);
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({want, cap, 16}));
+// A window's values when one node is left.  Over buckets: planes t = 0.. with
+// weight 2^t, then R with weight 1.  Over groups (glen > 0): T with weight 1,
+// planes t with weight 2^(glen + t), then R, which has no part.
+struct FinWin {
+    uint32_t start;
+    uint32_t v;
+    uint32_t glen_log;
+};
+constexpr uint32_t kFinThreads = 128;  // 32 quads: v <= 25 values (c <= 24)
+
+__global__ void __launch_bounds__(kFinThreads) k_tree_finish(const Xyzz* __restrict__ in,
+                                                             const FinWin* __restrict__ wins, Xyzz* __restrict__ out) {
+    __shared__ Xyzz sm[kFinThreads / 4];
+    const FinWin w = wins[blockIdx.x];
+    const uint32_t i = threadIdx.x >> 2;
+    Fp acc = fp_zero();
+    uint32_t shift = 0;
+    if (w.glen_log == 0) {
+        if (i < w.v) acc = quad_load(&in[w.start + i]);
+        if (i + 1 < w.v) shift = i;
+    } else if (i + 1 < w.v) {
+        acc = quad_load(&in[w.start + i]);
+        if (i > 0) shift = w.glen_log + i - 1;
+    }
+    for (uint32_t k = 0; __any_sync(0xffffffffu, k < shift); k++) {
+        const Fp d = quad_dbl(acc);
+        acc = fp_select(k < shift, d, acc);
+    }
+    quad_store(&sm[i], acc);
+    __syncthreads();
+    for (uint32_t off = kFinThreads / 8; off > 0; off >>= 1) {
+        if ((i & ~7u) < off) {
+            const Fp r = quad_add(quad_load(&sm[i]), i < off ? quad_load(&sm[i + off]) : fp_zero());
+            __syncwarp();
+            if (i < off) quad_store(&sm[i], r);
+        }
+        __syncthreads();
+    }
+    if (i == 0) quad_store(&out[blockIdx.x], quad_load(&sm[0]));
 }
 
-// steps 1-3 on `st`.  partial holds slots * split plane partials and may be
-// q itself when split == 1; q holds slots plane sums.  Returns the launch
-// error, if any; adds the launches to *launches when given.
-cudaError_t launch_reduce(const BucketSets& sets, const WinDev* d_wins, uint32_t n_wins, uint64_t groups,
-                          uint64_t slots, uint32_t split, Xyzz* run, Xyzz* tot, Xyzz* partial, Xyzz* q, Xyzz* wsum,
+// One window of a reduction: its buckets' keys
+struct Window {
+    uint32_t key_start;
+    uint32_t log_nb;
+};
+
+// The launches of one reduction and their tables
+struct ReducePlan {
+    uint32_t n_wins = 0;
+    uint32_t total_groups = 0;        // running-sum groups, 0: the tree starts at the buckets
+    std::vector<GroupWin> group;
+    std::vector<TreeWin> tree;        // every launch's table, back to back
+    struct Launch {
+        uint32_t first, count, blocks, threads;
+    };
+    std::vector<Launch> launches;
+    std::vector<FinWin> fin;
+    uint64_t arena = 0;  // points: the groups' pairs, then every launch's values
+    size_t table_bytes() const {
+        return group.size() * sizeof(GroupWin) + tree.size() * sizeof(TreeWin) + fin.size() * sizeof(FinWin);
+    }
+    void pack(void* dst) const {
+        char* p = static_cast<char*>(dst);
+        std::memcpy(p, group.data(), group.size() * sizeof(GroupWin));
+        p += group.size() * sizeof(GroupWin);
+        std::memcpy(p, tree.data(), tree.size() * sizeof(TreeWin));
+        p += tree.size() * sizeof(TreeWin);
+        std::memcpy(p, fin.data(), fin.size() * sizeof(FinWin));
+    }
+};
+
+// glen_log 0: the tree starts at the buckets
+ReducePlan plan_reduce(const std::vector<Window>& wins, uint32_t glen_log) {
+    ReducePlan p;
+    p.n_wins = (uint32_t)wins.size();
+    struct State {
+        uint32_t start, log_nodes, v, glen;
+    };
+    std::vector<State> st;
+    for (const Window& w : wins) {
+        if (glen_log) {
+            const uint32_t g = std::min(glen_log, w.log_nb);
+            p.group.push_back({w.key_start, p.total_groups, g});
+            st.push_back({2 * p.total_groups, w.log_nb - g, 2, g});
+            p.total_groups += 1u << (w.log_nb - g);
+        } else {
+            st.push_back({w.key_start, w.log_nb, 1, 0});
+        }
+    }
+    p.arena = 2 * (uint64_t)p.total_groups;
+    bool over_leaves = glen_log == 0;
+    for (;;) {
+        const uint32_t at = (uint32_t)p.tree.size();
+        uint32_t blocks = 0, most = 0;
+        for (State& s : st) {
+            if (s.log_nodes == 0) continue;
+            // as many heights as fit, seven over single buckets: 32 quads then
+            // have work for the first four of them.  Measured (MSM of 1000003
+            // points, 524288 buckets): 6 heights with 32 / 64 quads 7.55 /
+            // 8.29 ms per call, 7 with 32 / 64 7.42 / 7.79, 8 with 32 / 64
+            // 7.40 / 7.59; 65536 points: all within 3 %.
+            uint32_t b = 0;
+            while (b < s.log_nodes && (s.v << (b + 1)) <= kTreePoints && !(s.v == 1 && b == 7)) b++;
+            TreeWin t{blocks, s.start, (uint32_t)p.arena, s.v, b};
+            const uint32_t n = 1u << (s.log_nodes - b);
+            most = std::max(most, s.v << (b - 1));
+            blocks += n;
+            s.start = (uint32_t)p.arena;
+            s.v += b;
+            s.log_nodes -= b;
+            p.arena += (uint64_t)n * s.v;
+            p.tree.push_back(t);
+        }
+        if (p.tree.size() == at) break;
+        p.launches.push_back({at, (uint32_t)p.tree.size() - at, blocks, over_leaves || most <= 32 ? 128u : 256u});
+        over_leaves = false;
+    }
+    for (const State& s : st) p.fin.push_back({s.start, s.v, s.glen});
+    return p;
+}
+
+// Total buckets from which running sums over groups come first: the tree from
+// the buckets is faster at 1.6 M buckets (commitment batch of 24 items over a
+// window table: 25.0 ms per call against 26.0 with groups), the groups at 6.8 M
+// (2^24 points: 92.0 against 94.0).
+constexpr uint64_t kTreeKeys = 1u << 22;
+
+// log2 of the buckets per running-sum group of a call with `keys` buckets in
+// `sets` sets (0: none, the tree starts at the buckets)
+uint32_t reduce_group_log(uint64_t keys, uint32_t sets) {
+    if (sets == 1 && keys < kTreeKeys) return 0;
+    uint32_t g = 2;
+    while (g < 6 && (keys >> (g + 1)) >= 32768) g++;
+    return g;
+}
+
+// The launches of `p` on `st`.  d_tab: its packed tables; arena: p.arena
+// points.  Returns the launch error, if any; adds the launches to *launches
+// when given.
+cudaError_t launch_reduce(const ReducePlan& p, const BucketSets& sets, const void* d_tab, Xyzz* arena, Xyzz* wsum,
                           uint64_t* launches, cudaStream_t st) {
-    k_group_sums<<<(uint32_t)((groups + kReduceThreads - 1) / kReduceThreads), kReduceThreads, 0, st>>>(
-        sets, d_wins, n_wins, (uint32_t)groups, run, tot);
-    k_plane_sums<<<(uint32_t)(slots * split), kReduceThreads, kReduceThreads * sizeof(Xyzz), st>>>(
-        run, tot, d_wins, n_wins, split, split == 1 ? q : partial);
-    uint64_t n = 3;
-    if (split > 1) {
-        k_plane_merge<<<(uint32_t)((slots + 63) / 64), 64, 0, st>>>(partial, (uint32_t)slots, split, q);
+    const GroupWin* d_group = static_cast<const GroupWin*>(d_tab);
+    const TreeWin* d_tree = reinterpret_cast<const TreeWin*>(d_group + p.group.size());
+    const FinWin* d_fin = reinterpret_cast<const FinWin*>(d_tree + p.tree.size());
+    uint64_t n = 1;
+    if (p.total_groups) {
+        k_group_sums<<<(p.total_groups + kReduceThreads - 1) / kReduceThreads, kReduceThreads, 0, st>>>(
+            sets, d_group, p.n_wins, p.total_groups, arena);
         n++;
     }
-    k_window_finish<<<(n_wins + 31) / 32, 32, 0, st>>>(q, d_wins, n_wins, wsum);
+    bool over_buckets = p.total_groups == 0;
+    for (const ReducePlan::Launch& l : p.launches) {
+        k_tree<<<l.blocks, l.threads, 0, st>>>(over_buckets ? sets.buckets[0] : arena,
+                                               over_buckets ? sets.offsets[0] : nullptr, d_tree + l.first, l.count,
+                                               arena);
+        over_buckets = false;
+        n++;
+    }
+    k_tree_finish<<<p.n_wins, kFinThreads, 0, st>>>(arena, d_fin, wsum);
     if (launches) *launches += n;
     return cudaGetLastError();
+}
+
+// the windows of one MSM, appended to `wins`
+void append_windows(const MsmShape& sh, uint64_t key_base, int windows, std::vector<Window>& wins) {
+    for (int w = 0; w < windows; w++)
+        wins.push_back({(uint32_t)(key_base + (uint64_t)w * sh.nb), (uint32_t)(sh.c - 1)});
 }
 
 Status scan_u32(Context* ctx, const uint32_t* in, uint32_t* out, uint32_t len, cudaStream_t st) {
@@ -692,7 +827,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         set_error("msm: window width must be in [5, 24]");
         return ERR_ARG;
     }
-    const MsmShape sh = make_shape(c, group_log_for(make_shape(c).keys));
+    const MsmShape sh = make_shape(c);
     const size_t entries_cap = (size_t)sh.windows * max_part;
     if (entries_cap >= 0xffffffffull) {
         set_error("msm: n * windows exceeds 2^32 entries");
@@ -705,7 +840,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
 
-    void *counts, *sorted, *partials, *owner, *run, *tot, *planes, *wsum;
+    void *counts, *sorted, *partials, *owner, *arena, *wsum;
     void *offsets[kMaxMsmParts] = {}, *buckets[kMaxMsmParts] = {};
     static const char* const kOffsetNames[kMaxMsmParts] = {"msm_offsets", "msm_offsets2", "msm_offsets3",
                                                             "msm_offsets4"};
@@ -724,24 +859,20 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     void *long_count, *long_list;
     MZK_TRY(ctx->ensure("msm_long_count", 64, &long_count));
     MZK_TRY(ctx->ensure("msm_long_list", (size_t)acc_threads * sizeof(uint2), &long_list));
-    std::vector<WinDev> wins;
-    uint64_t total_groups = 0, slots = 0;
-    append_windows(sh, 0, wins, total_groups, slots);
-    const uint32_t split = plane_split(slots, sh.groups, ctx->num_sms);
-    void *d_wins, *q;
-    MZK_TRY(ctx->ensure("msm_wins", wins.size() * sizeof(WinDev), &d_wins));
-    MZK_TRY(ctx->ensure("msm_run", total_groups * sizeof(Xyzz), &run));
-    MZK_TRY(ctx->ensure("msm_tot", total_groups * sizeof(Xyzz), &tot));
-    MZK_TRY(ctx->ensure("msm_planes", slots * split * sizeof(Xyzz), &planes));
-    MZK_TRY(ctx->ensure("msm_q", slots * sizeof(Xyzz), &q));
+    std::vector<Window> wins;
+    append_windows(sh, 0, sh.windows, wins);
+    const ReducePlan plan = plan_reduce(wins, reduce_group_log(sh.keys, (uint32_t)n_parts));
+    void* d_tab;
+    MZK_TRY(ctx->ensure("msm_wins", plan.table_bytes(), &d_tab));
+    MZK_TRY(ctx->ensure("msm_arena", plan.arena * sizeof(Xyzz), &arena));
     MZK_TRY(ctx->ensure("msm_wsum", (size_t)sh.windows * sizeof(Xyzz), &wsum));
     // pinned staging: window sums and the parts' entry counts (read back),
-    // then the window table (uploaded without the sync a pageable copy implies)
+    // then the reduction's tables (uploaded without the sync a pageable copy implies)
     void* host_wsum;
     const size_t tab_off = (size_t)sh.windows * sizeof(Xyzz) + 64;
-    MZK_TRY(ctx->ensure_pinned(tab_off + wins.size() * sizeof(WinDev), &host_wsum));
-    WinDev* host_tab = reinterpret_cast<WinDev*>(static_cast<char*>(host_wsum) + tab_off);
-    std::memcpy(host_tab, wins.data(), wins.size() * sizeof(WinDev));
+    MZK_TRY(ctx->ensure_pinned(tab_off + plan.table_bytes(), &host_wsum));
+    void* host_tab = static_cast<char*>(host_wsum) + tab_off;
+    plan.pack(host_tab);
     uint32_t* host_entries =
         reinterpret_cast<uint32_t*>(static_cast<char*>(host_wsum) + (size_t)sh.windows * sizeof(Xyzz));
 
@@ -749,7 +880,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     const Affine* ba = static_cast<const Affine*>(d_bases);
     const int pt_threads = 256;
 
-    MZK_CUDA_CHECK(cudaMemcpyAsync(d_wins, host_tab, wins.size() * sizeof(WinDev), cudaMemcpyHostToDevice, st));
+    MZK_CUDA_CHECK(cudaMemcpyAsync(d_tab, host_tab, plan.table_bytes(), cudaMemcpyHostToDevice, st));
     for (int p = 0; p < n_parts; p++) {
         const MsmPart& part = parts[p];
         const size_t np = part.end - part.begin;
@@ -783,10 +914,11 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         MZK_TRY(ctx->phase_end(st));
         MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
         MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-        k_fixup<<<acc_blocks, kAccThreads, 0, st>>>(off, sh.keys, (const Xyzz*)partials, (const int*)owner,
-                                                   (Xyzz*)buckets[p], (uint32_t*)long_count, (uint2*)long_list);
+        k_fixup<<<acc_blocks * 4, kReduceThreads, 0, st>>>(off, sh.keys, acc_threads, (const Xyzz*)partials,
+                                                          (const int*)owner, (Xyzz*)buckets[p],
+                                                          (uint32_t*)long_count, (uint2*)long_list);
         MZK_LAUNCH_CHECK(ctx);
-        k_fixup_long<<<ctx->num_sms * 2, kReduceThreads, kReduceThreads * sizeof(Xyzz), st>>>(
+        k_fixup_long<<<ctx->num_sms * 2, kLongThreads, 0, st>>>(
             (const int*)owner, (const Xyzz*)partials, (const uint32_t*)long_count, (const uint2*)long_list,
             (Xyzz*)buckets[p]);
         MZK_LAUNCH_CHECK(ctx);
@@ -800,9 +932,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         sets.buckets[p] = (const Xyzz*)buckets[p];
         sets.offsets[p] = (const uint32_t*)offsets[p];
     }
-    MZK_CUDA_CHECK(launch_reduce(sets, (const WinDev*)d_wins, (uint32_t)wins.size(),
-                                 total_groups, slots, split, (Xyzz*)run, (Xyzz*)tot, (Xyzz*)planes, (Xyzz*)q,
-                                 (Xyzz*)wsum, &ctx->launches, st));
+    MZK_CUDA_CHECK(launch_reduce(plan, sets, d_tab, (Xyzz*)arena, (Xyzz*)wsum, &ctx->launches, st));
     MZK_TRY(ctx->phase_end(st));
     MZK_CUDA_CHECK(cudaMemcpyAsync(host_wsum, wsum, (size_t)sh.windows * sizeof(Xyzz), cudaMemcpyDeviceToHost, st));
     MZK_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -955,19 +1085,11 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     }
     std::memset(out, 0, count * 18 * 8);
     std::vector<BatchItemDev> hi;
-    std::vector<WinDev> hw;
+    std::vector<Window> hw;
     std::vector<size_t> item_of;  // position in `items` of every device item
-    uint64_t points = 0, keys = 0, entries = 0, groups = 0, slots = 0;
-    uint32_t max_groups = 1;
+    uint64_t points = 0, keys = 0, entries = 0;
     int max_windows = 0;
-    // the group length follows the buckets of the whole batch
     auto uses_table = [&](uint64_t n) { return table && n >= table->min_n; };
-    uint64_t all_keys = 0;
-    for (size_t m = 0; m < count; m++)
-        if (items[m].n)
-            all_keys += uses_table(items[m].n) ? make_shape(table->c).nb
-                                                : make_shape(msm_window_for(ctx, items[m].n)).keys;
-    const int glen_log = group_log_for(all_keys);
     for (size_t m = 0; m < count; m++) {
         const BatchItem& it = items[m];
         if (it.n == 0) continue;
@@ -981,7 +1103,7 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
         }
         const bool fixed = uses_table(it.n);
         const int c = fixed ? table->c : msm_window_for(ctx, it.n);
-        const MsmShape sh = make_shape(c, glen_log);
+        const MsmShape sh = make_shape(c);
         BatchItemDev d;
         d.scalars = static_cast<const Fr*>(it.d_scalars);
         d.n = (uint32_t)it.n;
@@ -992,16 +1114,9 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
         d.nb = sh.nb;
         d.key_start = (uint32_t)keys;
         d.fixed = fixed ? 1u : 0u;
-        if (fixed) {  // one window row: every window's digits land in the same buckets
-            MsmShape one = sh;
-            one.windows = 1;
-            append_windows(one, keys, hw, groups, slots);
-            keys += sh.nb;
-        } else {
-            append_windows(sh, keys, hw, groups, slots);
-            keys += sh.keys;
-        }
-        max_groups = std::max(max_groups, sh.groups);
+        // fixed: one bucket set, every window's digits land in the same buckets
+        append_windows(sh, keys, fixed ? 1 : sh.windows, hw);
+        keys += fixed ? sh.nb : sh.keys;
         points += it.n;
         entries += (uint64_t)sh.windows * it.n;
         max_windows = std::max(max_windows, sh.windows);
@@ -1019,10 +1134,11 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
     const size_t n_wins = hw.size();
-    void *d_items, *d_wins, *counts, *offsets, *sorted, *buckets, *partials, *owner, *long_count, *long_list, *run, *tot,
-        *planes, *wsum;
+    const ReducePlan plan = plan_reduce(hw, reduce_group_log(keys, 1));
+    void *d_items, *d_tab, *counts, *offsets, *sorted, *buckets, *partials, *owner, *long_count, *long_list, *arena,
+        *wsum;
     MZK_TRY(ctx->ensure("batch_items", hi.size() * sizeof(BatchItemDev), &d_items));
-    MZK_TRY(ctx->ensure("batch_wins", n_wins * sizeof(WinDev), &d_wins));
+    MZK_TRY(ctx->ensure("batch_wins", plan.table_bytes(), &d_tab));
     MZK_TRY(ctx->ensure("msm_counts", (keys + 1) * 4, &counts));
     MZK_TRY(ctx->ensure("msm_offsets", (keys + 2) * 4, &offsets));
     MZK_TRY(ctx->ensure("msm_sorted", entries * 4, &sorted));
@@ -1033,24 +1149,19 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     MZK_TRY(ctx->ensure("msm_owner", (size_t)acc_threads * 4, &owner));
     MZK_TRY(ctx->ensure("msm_long_count", 64, &long_count));
     MZK_TRY(ctx->ensure("msm_long_list", (size_t)acc_threads * sizeof(uint2), &long_list));
-    MZK_TRY(ctx->ensure("msm_run", groups * sizeof(Xyzz), &run));
-    MZK_TRY(ctx->ensure("msm_tot", groups * sizeof(Xyzz), &tot));
-    const uint32_t split = plane_split(slots, max_groups, ctx->num_sms);
-    void* q;
-    MZK_TRY(ctx->ensure("msm_planes", slots * split * sizeof(Xyzz), &planes));
-    MZK_TRY(ctx->ensure("msm_q", slots * sizeof(Xyzz), &q));
+    MZK_TRY(ctx->ensure("msm_arena", plan.arena * sizeof(Xyzz), &arena));
     MZK_TRY(ctx->ensure("msm_wsum", n_wins * sizeof(Xyzz), &wsum));
-    // pinned staging: window sums (read back), then the item and window tables
+    // pinned staging: window sums (read back), then the item table and the reduction's tables
     void* host_wsum;
     const size_t items_off = n_wins * sizeof(Xyzz) + 64;
     const size_t wins_off = items_off + ((hi.size() * sizeof(BatchItemDev) + 255) & ~(size_t)255);
-    MZK_TRY(ctx->ensure_pinned(wins_off + n_wins * sizeof(WinDev), &host_wsum));
+    MZK_TRY(ctx->ensure_pinned(wins_off + plan.table_bytes(), &host_wsum));
     char* staging = static_cast<char*>(host_wsum);
     std::memcpy(staging + items_off, hi.data(), hi.size() * sizeof(BatchItemDev));
-    std::memcpy(staging + wins_off, hw.data(), n_wins * sizeof(WinDev));
+    plan.pack(staging + wins_off);
     MZK_CUDA_CHECK(cudaMemcpyAsync(d_items, staging + items_off, hi.size() * sizeof(BatchItemDev),
                                    cudaMemcpyHostToDevice, st));
-    MZK_CUDA_CHECK(cudaMemcpyAsync(d_wins, staging + wins_off, n_wins * sizeof(WinDev), cudaMemcpyHostToDevice, st));
+    MZK_CUDA_CHECK(cudaMemcpyAsync(d_tab, staging + wins_off, plan.table_bytes(), cudaMemcpyHostToDevice, st));
 
     const uint32_t n_items = (uint32_t)hi.size();
     const int pt_threads = 256;
@@ -1084,19 +1195,18 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
     MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-    k_fixup<<<acc_blocks, kAccThreads, 0, st>>>((const uint32_t*)offsets, (uint32_t)keys, (const Xyzz*)partials,
-                                               (const int*)owner, (Xyzz*)buckets, (uint32_t*)long_count,
-                                               (uint2*)long_list);
+    k_fixup<<<acc_blocks * 4, kReduceThreads, 0, st>>>((const uint32_t*)offsets, (uint32_t)keys, acc_threads,
+                                                      (const Xyzz*)partials, (const int*)owner, (Xyzz*)buckets,
+                                                      (uint32_t*)long_count, (uint2*)long_list);
     MZK_LAUNCH_CHECK(ctx);
-    k_fixup_long<<<ctx->num_sms * 2, kReduceThreads, kReduceThreads * sizeof(Xyzz), st>>>(
+    k_fixup_long<<<ctx->num_sms * 2, kLongThreads, 0, st>>>(
         (const int*)owner, (const Xyzz*)partials, (const uint32_t*)long_count, (const uint2*)long_list,
         (Xyzz*)buckets);
     MZK_LAUNCH_CHECK(ctx);
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
     const BucketSets sets{{(const Xyzz*)buckets}, {(const uint32_t*)offsets}, 1};
-    MZK_CUDA_CHECK(launch_reduce(sets, (const WinDev*)d_wins, (uint32_t)n_wins, groups, slots, split, (Xyzz*)run,
-                                 (Xyzz*)tot, (Xyzz*)planes, (Xyzz*)q, (Xyzz*)wsum, &ctx->launches, st));
+    MZK_CUDA_CHECK(launch_reduce(plan, sets, d_tab, (Xyzz*)arena, (Xyzz*)wsum, &ctx->launches, st));
     MZK_TRY(ctx->phase_end(st));
     MZK_CUDA_CHECK(cudaMemcpyAsync(host_wsum, wsum, n_wins * sizeof(Xyzz), cudaMemcpyDeviceToHost, st));
     MZK_CUDA_CHECK(cudaStreamSynchronize(st));
@@ -1171,15 +1281,15 @@ constexpr size_t kNaSortedOff = kNaOffsetsOff + align256((kNaKeys + 2) * 4);
 constexpr size_t kNaBucketsOff = kNaSortedOff + align256(kNaMaxWindows * kNoAllocMaxN * 4);
 constexpr size_t kNaPartialsOff = kNaBucketsOff + align256(kNaKeys * sizeof(Xyzz));
 constexpr size_t kNaOwnerOff = kNaPartialsOff + align256(kNaAccThreads * 2 * sizeof(Xyzz));
-constexpr size_t kNaRunOff = kNaOwnerOff + align256(kNaAccThreads * 4);
-// running-sum groups of 2^kNoAllocGroupLog buckets (c >= 8)
-constexpr int kNoAllocGroupLog = 4;
-constexpr size_t kNaTotOff = kNaRunOff + align256((kNaKeys >> kNoAllocGroupLog) * sizeof(Xyzz));
-constexpr size_t kNaPlanesOff = kNaTotOff + align256((kNaKeys >> kNoAllocGroupLog) * sizeof(Xyzz));
-constexpr size_t kNaWsumOff = kNaPlanesOff + align256(kNaMaxWindows * 8 * sizeof(Xyzz));
+constexpr size_t kNaArenaOff = kNaOwnerOff + align256(kNaAccThreads * 4);
+// the reduction tree's values over the widest key count: a node of 64 buckets
+// leaves 7 values, and the one or two launches above it far fewer
+constexpr size_t kNaArenaPoints = kNaKeys / 64 * 7 + kNaMaxWindows * 32;
+constexpr size_t kNaTabBytes = kNaMaxWindows * (4 * sizeof(TreeWin) + sizeof(FinWin));
+constexpr size_t kNaWsumOff = kNaArenaOff + align256(kNaArenaPoints * sizeof(Xyzz));
 constexpr size_t kNaScanOff = kNaWsumOff + align256(kNaMaxWindows * sizeof(Xyzz));
 constexpr size_t kNaWinsOff = kNaScanOff + align256(64 * 4);
-constexpr size_t kNaLongOff = kNaWinsOff + align256(kNaMaxWindows * sizeof(WinDev));
+constexpr size_t kNaLongOff = kNaWinsOff + align256(kNaTabBytes);
 constexpr size_t kNaBytes = kNaLongOff + align256(16 + kNaAccThreads * sizeof(uint2));
 
 // The scratch itself.  Host code must not use this name as a device address:
@@ -1248,16 +1358,14 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
                              uint64_t* out18, cudaStream_t st) {
     int c = msm_pick_window(n);
     c = c < kNoAllocMinC ? kNoAllocMinC : (c > kNoAllocMaxC ? kNoAllocMaxC : c);
-    const MsmShape sh = make_shape(c, kNoAllocGroupLog);
+    const MsmShape sh = make_shape(c);
     uint32_t* counts = reinterpret_cast<uint32_t*>(base + kNaCountsOff);
     uint32_t* offsets = reinterpret_cast<uint32_t*>(base + kNaOffsetsOff);
     uint32_t* sorted = reinterpret_cast<uint32_t*>(base + kNaSortedOff);
     Xyzz* buckets = reinterpret_cast<Xyzz*>(base + kNaBucketsOff);
     Xyzz* partials = reinterpret_cast<Xyzz*>(base + kNaPartialsOff);
     int* owner = reinterpret_cast<int*>(base + kNaOwnerOff);
-    Xyzz* run = reinterpret_cast<Xyzz*>(base + kNaRunOff);
-    Xyzz* tot = reinterpret_cast<Xyzz*>(base + kNaTotOff);
-    Xyzz* planes = reinterpret_cast<Xyzz*>(base + kNaPlanesOff);
+    Xyzz* arena = reinterpret_cast<Xyzz*>(base + kNaArenaOff);
     Xyzz* wsum = reinterpret_cast<Xyzz*>(base + kNaWsumOff);
     uint32_t* scan_sums = reinterpret_cast<uint32_t*>(base + kNaScanOff);
 
@@ -1279,22 +1387,24 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
     uint32_t* long_count = reinterpret_cast<uint32_t*>(base + kNaLongOff);
     uint2* long_list = reinterpret_cast<uint2*>(base + kNaLongOff + 16);
     MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-    k_fixup<<<kNoAllocAccBlocks, kAccThreads, 0, st>>>(offsets, sh.keys, partials, owner, buckets, long_count,
-                                                       long_list);
+    k_fixup<<<kNoAllocAccBlocks * 4, kReduceThreads, 0, st>>>(offsets, sh.keys, (uint32_t)kNaAccThreads, partials,
+                                                             owner, buckets, long_count, long_list);
     MZK_CUDA_CHECK(cudaGetLastError());
-    k_fixup_long<<<kNoAllocAccBlocks, kReduceThreads, kReduceThreads * sizeof(Xyzz), st>>>(owner, partials,
-                                                                                          long_count, long_list,
-                                                                                          buckets);
+    k_fixup_long<<<kNoAllocAccBlocks, kLongThreads, 0, st>>>(owner, partials, long_count, long_list, buckets);
     MZK_CUDA_CHECK(cudaGetLastError());
-    // window table (a copy from pageable memory is staged before the call returns)
-    std::vector<WinDev> wins;
-    uint64_t total_groups = 0, slots = 0;
-    append_windows(sh, 0, wins, total_groups, slots);
-    WinDev* d_wins = reinterpret_cast<WinDev*>(base + kNaWinsOff);
-    MZK_CUDA_CHECK(cudaMemcpyAsync(d_wins, wins.data(), wins.size() * sizeof(WinDev), cudaMemcpyHostToDevice, st));
+    // the reduction's tables (a copy from pageable memory is staged before the call returns)
+    std::vector<Window> wins;
+    append_windows(sh, 0, sh.windows, wins);
+    const ReducePlan plan = plan_reduce(wins, 0);
+    if (plan.arena > kNaArenaPoints || plan.table_bytes() > kNaTabBytes) {
+        set_error("mzk_msm_g1_noalloc: the reduction does not fit the fixed scratch");
+        return ERR_STATE;
+    }
+    unsigned char tab[kNaTabBytes];
+    plan.pack(tab);
+    MZK_CUDA_CHECK(cudaMemcpyAsync(base + kNaWinsOff, tab, plan.table_bytes(), cudaMemcpyHostToDevice, st));
     const BucketSets sets{{buckets}, {offsets}, 1};
-    MZK_CUDA_CHECK(launch_reduce(sets, d_wins, (uint32_t)wins.size(), total_groups, slots, 1, run, tot, planes, planes,
-                                 wsum, nullptr, st));
+    MZK_CUDA_CHECK(launch_reduce(plan, sets, base + kNaWinsOff, arena, wsum, nullptr, st));
     // window sums to host memory owned by this function (no pinned allocation)
     host::Xyzz6 hs[kNaMaxWindows];
     MZK_CUDA_CHECK(cudaMemcpyAsync(hs, wsum, (size_t)sh.windows * sizeof(Xyzz), cudaMemcpyDeviceToHost, st));

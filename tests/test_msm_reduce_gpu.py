@@ -1,0 +1,72 @@
+"""The bucket reduction of an MSM (partial sums of cut buckets, the tree over a
+window's buckets, running sums over groups of them where buckets are many)
+against the oracle's plain double-and-add sum, bit-exact.
+
+The inputs drive every additions' special cases: buckets that hold the same
+point (doublings all the way up the tree), opposite points (the tree meets
+infinity), empty buckets, and buckets cut into few and into many chunks.
+"""
+import numpy as np
+import pytest
+
+from _loader import load
+from oracle import oracle as O
+
+mzk = load()
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = mzk.Context(0)
+    yield c
+    c.close()
+
+
+def small_scalars(values):
+    """Montgomery forms of small whole numbers, by repeated doubling and adding."""
+    one = O.fr_const(0)
+    out = np.zeros((len(values), 4), np.uint64)
+    for i, v in enumerate(values):
+        acc = np.zeros(4, np.uint64)
+        for bit in bin(int(v))[2:]:
+            acc = O.fr_op("add", acc, acc)
+            if bit == "1":
+                acc = O.fr_op("add", acc, one)
+        out[i] = acc
+    return out
+
+
+def negated(p):
+    q = p.copy()
+    q[6:] = O.fp_op("sub", np.zeros(6, np.uint64), p[6:])
+    return q
+
+
+def inputs(kind):
+    g = O.gen_bases(11, 400)
+    if kind == "one point":              # every bucket the same point
+        s, b = small_scalars(range(1, 301)), np.repeat(g[:1], 300, axis=0)
+    elif kind == "opposite points":      # neighbouring buckets cancel pairwise
+        s = small_scalars([1 + i // 2 for i in range(300)])
+        b = np.stack([g[0] if i % 4 in (0, 3) else negated(g[0]) for i in range(300)])
+    elif kind == "cut buckets":          # spans of 1 .. 300 chunks, both sides of the short-span limit
+        runs = [1, 2, 3, 11, 12, 13, 14, 15, 63, 64, 65, 66, 129, 300]
+        s = small_scalars([7 * (i + 1) for i, r in enumerate(runs) for _ in range(r)])
+        b = np.concatenate([g[:r] for r in runs])
+    else:
+        s, b = O.rand_fr(13, 400), g
+    return s, np.ascontiguousarray(b)
+
+
+# 5: the narrowest window; 8 and 9: one block of the tree and two; 13, 16, 18: several launches; 20: groups first
+@pytest.mark.parametrize("c", [5, 8, 9, 13, 16, 18, 20])
+@pytest.mark.parametrize("kind", ["one point", "opposite points", "cut buckets", "uniform"])
+def test_reduction_matches_the_plain_sum(ctx, c, kind):
+    s, b = inputs(kind)
+    ctx.set_msm_window(c)
+    try:
+        got = ctx.msm_best(s, b)
+    finally:
+        ctx.set_msm_window(0)
+    assert np.array_equal(mzk.affine(got), O.msm_naive(s, b))
