@@ -167,8 +167,9 @@ __device__ __forceinline__ void scatter_group(const uint32_t (&key)[kScatterWind
 // window's slice of the sorted array (4n bytes: 67 MB at 2^24, inside the
 // 126 MB L2), so the scattered 4-byte writes merge into whole sectors in L2
 // instead of each costing a DRAM sector read and write.
-__global__ void k_scatter_window(const uint32_t* __restrict__ digits_w, size_t n, uint32_t* __restrict__ cursor,
-                                 uint32_t* __restrict__ sorted) {
+__global__ void k_scatter_window(const uint32_t* __restrict__ digits, size_t n, uint32_t w0,
+                                 uint32_t* __restrict__ cursor, uint32_t* __restrict__ sorted) {
+    const uint32_t* __restrict__ digits_w = digits + (size_t)(w0 + blockIdx.y) * n;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -183,6 +184,17 @@ __global__ void k_scatter_window(const uint32_t* __restrict__ digits_w, size_t n
         slot = __shfl_sync(0xffffffffu, slot, leader);
         if (key != kNoKey) sorted[slot + (uint32_t)__popc(peers & lt_mask)] = (uint32_t)i | (d & 0x80000000u);
     }
+}
+
+// Windows scattered by one launch of k_scatter_window(_batch): as many as keep
+// their entries (4 bytes each) within a quarter of L2.  A launch per window
+// costs 3.5 us whatever its size: 1000 points (32 windows) 744 -> 620 us per
+// call, a proof of 2^14 rows 7.30 -> 6.75 ms.  At 10^6 points one launch of 8
+// windows or 16 measures the same (7.37 ms, 7.45 window by window).
+constexpr size_t kScatterBytes = 32u << 20;
+
+uint32_t scatter_together(size_t windows, size_t points) {
+    return (uint32_t)std::min(windows, std::max<size_t>(1, kScatterBytes / (points * 4)));
 }
 
 __global__ void k_scatter(const Fr* __restrict__ scalars, size_t n, int c, int windows, uint32_t nb,
@@ -324,15 +336,21 @@ __device__ __forceinline__ void chunk_range(uint32_t total, uint32_t t, uint32_t
 // One flat loop over the chunk, so every thread of a warp runs the same number
 // of additions whatever its bucket boundaries; a boundary only costs a short
 // divergent flush.
+// The chunks that a cut bucket starts in, queued for k_fixup
+struct Owners {
+    uint32_t* count;
+    uint2* list;  // (chunk, bucket key)
+};
+
 __device__ __forceinline__ void flush_bucket(const Xyzz& acc, uint32_t k, uint32_t seg_lo, uint32_t seg_hi, uint32_t s,
-                                             uint32_t e, uint32_t t, Xyzz* buckets, Xyzz* partials, int* owner_key) {
+                                             uint32_t e, uint32_t t, Xyzz* buckets, Xyzz* partials, const Owners& own) {
     if (seg_lo >= s && seg_hi <= e) {
         store_xyzz(&buckets[k], acc);
     } else if (seg_lo < s) {
         store_xyzz(&partials[2 * (size_t)t], acc);
     } else {
         store_xyzz(&partials[2 * (size_t)t + 1], acc);
-        owner_key[t] = (int)k;
+        own.list[atomicAdd(own.count, 1u)] = make_uint2(t, k);
     }
 }
 
@@ -340,13 +358,12 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
                                                             const uint32_t* __restrict__ sorted,
                                                             const uint32_t* __restrict__ offsets, uint32_t keys,
                                                             Xyzz* __restrict__ buckets, Xyzz* __restrict__ partials,
-                                                            int* __restrict__ owner_key) {
+                                                            const Owners own) {
     const uint32_t nthreads = gridDim.x * blockDim.x;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t total = offsets[keys];
     uint32_t s, e;
     chunk_range(total, t, nthreads, s, e);
-    owner_key[t] = -1;
     if (s >= e) return;
     uint32_t k = find_key(offsets, keys, s);
     uint32_t seg_lo = offsets[k], seg_hi = offsets[k + 1];
@@ -362,7 +379,7 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
     Affine nxt = load_affine(bases, ent & 0x7fffffffu);
     for (uint32_t j = s; j < e; j++) {
         if (j == seg_hi) {
-            flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, owner_key);
+            flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, own);
             xyzz_set_inf(acc);
             k++;
             seg_lo = seg_hi;
@@ -392,43 +409,127 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
             xyzz_add_affine_fast(acc, p);
         }
     }
-    flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, owner_key);
+    flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, own);
 }
 
-// A cut bucket is finished by the chunk where it starts: one quad of lanes per
-// chunk, since the additions of a span are a serial chain.  A bucket spanning
-// many chunks (a heavy bucket: scalars 0/1, a nearly empty top window) is
-// queued for k_fixup_long, whose 64 quads take ~30 us for any span up to 65: the
-// chain of 12 additions that a quad still takes itself costs ~55.  Device time
-// of both kernels, quads against lanes: proof of 2^14 rows (6 calls) 2.51 ->
-// 1.70 ms, 2^16 points 150 -> 70 us.
+// The same walk with one quad of lanes per chunk, for inputs too small to fill
+// the GPU with lanes (accumulate_quad_blocks): bound by the latency of the
+// additions, which a quad finishes in less than half the time.  An affine
+// point enters quad_add with ZZ = ZZZ = 1.
+__global__ void __launch_bounds__(kAccThreads) k_accumulate_quads(const Affine* __restrict__ bases,
+                                                                  const uint32_t* __restrict__ sorted,
+                                                                  const uint32_t* __restrict__ offsets, uint32_t keys,
+                                                                  Xyzz* __restrict__ buckets,
+                                                                  Xyzz* __restrict__ partials, const Owners own) {
+    const uint32_t chunks = (gridDim.x * blockDim.x) >> 2;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const uint32_t q = threadIdx.x & 3, base = threadIdx.x & 28;
+    const uint32_t total = offsets[keys];
+    const uint32_t len = (total + chunks - 1) / chunks;
+    uint32_t s, e;
+    chunk_range(total, t, chunks, s, e);
+    uint32_t k = 0, seg_lo = 0, seg_hi = 0;
+    if (s < e) {
+        k = find_key(offsets, keys, s);
+        seg_lo = offsets[k];
+        seg_hi = offsets[k + 1];
+    }
+    // lanes 0 and 1 load x and y, one entry ahead
+    auto load = [&](uint32_t ent) {
+        const uint4* src = reinterpret_cast<const uint4*>(bases + (ent & 0x7fffffffu)) + 3 * q;
+        Fp r = fp_one();
+        if (q < 2) {
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                const uint4 v = __ldg(src + i);
+                r.l[4 * i] = v.x;
+                r.l[4 * i + 1] = v.y;
+                r.l[4 * i + 2] = v.z;
+                r.l[4 * i + 3] = v.w;
+            }
+        }
+        return r;
+    };
+    auto flush = [&](const Fp& acc) {
+        if (seg_lo >= s && seg_hi <= e) {
+            quad_store(&buckets[k], acc);
+        } else if (seg_lo < s) {
+            quad_store(&partials[2 * (size_t)t], acc);
+        } else {
+            quad_store(&partials[2 * (size_t)t + 1], acc);
+            if (q == 0) own.list[atomicAdd(own.count, 1u)] = make_uint2(t, k);
+        }
+    };
+    Fp acc = fp_zero(), nxt = fp_zero();
+    uint32_t ent = 0;
+    if (s < e) {
+        ent = __ldg(sorted + s);
+        nxt = load(ent);
+    }
+    for (uint32_t i = 0; i < len; i++) {  // the same count for every quad
+        const uint32_t j = s + i;
+        const bool on = j < e;
+        if (on && j == seg_hi) {
+            flush(acc);
+            acc = fp_zero();
+            do {  // past empty buckets
+                k++;
+                seg_lo = seg_hi;
+                seg_hi = offsets[k + 1];
+            } while (seg_hi <= j);
+        }
+        Fp p = nxt;
+        const uint32_t cur = ent;
+        if (j + 1 < e) {
+            ent = __ldg(sorted + j + 1);
+            nxt = load(ent);
+        }
+        const uint32_t z = (__ballot_sync(0xffffffffu, fp_is_zero_raw(p)) >> base) & 3u;  // x and y both zero: infinity
+        p = fp_select(q == 1 && (cur >> 31) != 0, fp_neg(p), p);
+        acc = quad_add(acc, fp_select(on && z != 3u, p, fp_zero()));
+    }
+    if (s < e) flush(acc);
+}
+
+// A cut bucket is finished by one quad of lanes, since the additions of its
+// span are a serial chain.  The buckets come from a list that the accumulation
+// made, so that the quads of a warp all have one: where a bucket spans many
+// chunks few chunks start one, and walking the chunks instead left most quads
+// idle (proof of 2^14 rows, six calls: 699 us).  A bucket spanning many chunks
+// (a heavy bucket: scalars 0/1, a nearly empty top window) is queued for
+// k_fixup_long, whose 64 quads take ~30 us for any span up to 65: the chain of
+// 12 additions that a quad still takes itself costs ~55.
 constexpr uint32_t kShortSpan = 12;
 
-// quads beyond `chunks` and chunks without an owner add nothing (whole warps
-// stay together in quad_add)
+struct LongSpans {
+    uint32_t* count;
+    uint4* list;  // (first chunk, last chunk, bucket key)
+};
+
 __global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __restrict__ offsets, uint32_t keys,
                                                           uint32_t chunks, const Xyzz* __restrict__ partials,
-                                                          const int* __restrict__ owner_key, Xyzz* __restrict__ buckets,
-                                                          uint32_t* __restrict__ long_count,
-                                                          uint2* __restrict__ long_list) {
-    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
-    const int k = t < chunks ? owner_key[t] : -1;
-    uint32_t last = t;
+                                                          const Owners own, Xyzz* __restrict__ buckets,
+                                                          const LongSpans spans) {
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, n = *own.count;
+    if ((i & ~7u) >= n) return;  // the whole warp
+    bool mine = i < n;
+    uint32_t u = 1, last = 0, k = 0;
     Fp acc = fp_zero();
-    bool mine = k >= 0;
     if (mine) {
-        const uint32_t total = offsets[keys];
-        const uint32_t len = (total + chunks - 1) / chunks;
+        const uint2 o = own.list[i];
+        const uint32_t t = o.x, total = offsets[keys], len = (total + chunks - 1) / chunks;
+        k = o.y;
         last = (offsets[k + 1] - 1) / len;
+        u = t + 1;
         if (last - t > kShortSpan) {
-            if ((threadIdx.x & 3) == 0) long_list[atomicAdd(long_count, 1u)] = make_uint2(t, last);
-            last = t;
+            if ((threadIdx.x & 3) == 0) spans.list[atomicAdd(spans.count, 1u)] = make_uint4(t, last, k, 0);
             mine = false;
+            last = t;
         } else {
             acc = quad_load(&partials[2 * (size_t)t + 1]);
         }
     }
-    for (uint32_t u = t + 1; __any_sync(0xffffffffu, u <= last); u++)
+    for (; __any_sync(0xffffffffu, u <= last); u++)
         acc = quad_add(acc, u <= last ? quad_load(&partials[2 * (size_t)u]) : fp_zero());
     if (mine) quad_store(&buckets[k], acc);
 }
@@ -437,17 +538,14 @@ __global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __rest
 // then the block's points are added pairwise
 constexpr int kLongThreads = 256;
 
-__global__ void __launch_bounds__(kLongThreads) k_fixup_long(const int* __restrict__ owner_key,
-                                                             const Xyzz* __restrict__ partials,
-                                                             const uint32_t* __restrict__ long_count,
-                                                             const uint2* __restrict__ long_list,
+__global__ void __launch_bounds__(kLongThreads) k_fixup_long(const Xyzz* __restrict__ partials, const LongSpans spans,
                                                              Xyzz* __restrict__ buckets) {
     constexpr uint32_t kQuads = kLongThreads / 4;
     __shared__ Xyzz sm[kQuads];
     const uint32_t quad = threadIdx.x >> 2;
-    for (uint32_t item = blockIdx.x; item < *long_count; item += gridDim.x) {
-        const uint2 tl = long_list[item];
-        const uint32_t t = tl.x, last = tl.y;
+    for (uint32_t item = blockIdx.x; item < *spans.count; item += gridDim.x) {
+        const uint4 sp = spans.list[item];
+        const uint32_t t = sp.x, last = sp.y;
         Fp acc = quad == 0 ? quad_load(&partials[2 * (size_t)t + 1]) : fp_zero();
         for (uint32_t u = t + 1 + quad; __any_sync(0xffffffffu, u <= last); u += kQuads)
             acc = quad_add(acc, u <= last ? quad_load(&partials[2 * (size_t)u]) : fp_zero());
@@ -460,7 +558,7 @@ __global__ void __launch_bounds__(kLongThreads) k_fixup_long(const int* __restri
             }
             __syncthreads();
         }
-        if (quad == 0) quad_store(&buckets[owner_key[t]], quad_load(&sm[0]));
+        if (quad == 0) quad_store(&buckets[sp.z], quad_load(&sm[0]));
         __syncthreads();
     }
 }
@@ -621,7 +719,7 @@ __global__ void __launch_bounds__(kFinThreads) k_tree_finish(const Xyzz* __restr
     }
     quad_store(&sm[i], acc);
     __syncthreads();
-    for (uint32_t off = kFinThreads / 8; off > 0; off >>= 1) {
+    for (uint32_t off = 1u << (31 - __clz(w.v - 1)); off > 0; off >>= 1) {  // w.v >= 2 values
         if ((i & ~7u) < off) {
             const Fp r = quad_add(quad_load(&sm[i]), i < off ? quad_load(&sm[i + off]) : fp_zero());
             __syncwarp();
@@ -761,6 +859,57 @@ void append_windows(const MsmShape& sh, uint64_t key_base, int windows, std::vec
         wins.push_back({(uint32_t)(key_base + (uint64_t)w * sh.nb), (uint32_t)(sh.c - 1)});
 }
 
+// Blocks of k_accumulate_quads for at most `entries` sorted entries, 0 where
+// one lane per chunk is faster.  A lane adds one point in ~12 us, a quad in ~5,
+// and a quarter as many chunks leave the cut buckets shorter spans: with up to
+// ~16 entries per quad that is faster than 1..4 per lane.  Per call, lanes
+// against quads: 1000 points (32000 entries) 620 -> 451 us, 4096 (119000
+// entries) 590 -> 525, 8192 (213000) 592 -> 635.  Two blocks of 128 per SM: with
+// one 470 us, with three 466 at 1000 points.
+constexpr uint64_t kQuadEntries = 150000;
+
+uint32_t accumulate_quad_blocks(const Context* ctx, uint64_t entries) {
+    return entries > kQuadEntries ? 0u : (uint32_t)ctx->num_sms * 2;
+}
+
+// The queues of an accumulation: both counters in 16 bytes, then the owners
+// and the long spans (at most one of each per chunk).
+struct Queues {
+    Owners own;
+    LongSpans spans;
+};
+constexpr size_t queue_bytes(size_t chunks) { return 16 + chunks * (sizeof(uint4) + sizeof(uint2)); }
+Queues queues_at(void* p, size_t chunks) {
+    uint32_t* counts = static_cast<uint32_t*>(p);
+    uint4* spans = reinterpret_cast<uint4*>(counts + 4);
+    return {{counts, reinterpret_cast<uint2*>(spans + chunks)}, {counts + 1, spans}};
+}
+
+// The bucket accumulation, by quads (quad_blocks > 0) or by lanes, and the
+// sums of the buckets that its chunks cut.  `queue` holds queue_bytes of the
+// lanes' grid, which is the larger one.  Returns the launch error, if any.
+cudaError_t launch_accumulate(const Affine* bases, const uint32_t* sorted, const uint32_t* offsets, uint32_t keys,
+                              Xyzz* buckets, Xyzz* partials, void* queue, uint32_t acc_blocks, uint32_t quad_blocks,
+                              cudaStream_t st) {
+    const Queues q = queues_at(queue, (size_t)acc_blocks * kAccThreads);
+    const cudaError_t e = cudaMemsetAsync(queue, 0, 16, st);
+    if (e != cudaSuccess) return e;
+    if (quad_blocks)
+        k_accumulate_quads<<<quad_blocks, kAccThreads, 0, st>>>(bases, sorted, offsets, keys, buckets, partials, q.own);
+    else
+        k_accumulate<<<acc_blocks, kAccThreads, 0, st>>>(bases, sorted, offsets, keys, buckets, partials, q.own);
+    return cudaGetLastError();
+}
+cudaError_t launch_fixup(const uint32_t* offsets, uint32_t keys, Xyzz* buckets, const Xyzz* partials, void* queue,
+                         uint32_t acc_blocks, uint32_t quad_blocks, uint32_t long_blocks, cudaStream_t st) {
+    const Queues q = queues_at(queue, (size_t)acc_blocks * kAccThreads);
+    const uint32_t chunks = quad_blocks ? quad_blocks * (kAccThreads / 4) : acc_blocks * kAccThreads;
+    k_fixup<<<chunks * 4 / kReduceThreads, kReduceThreads, 0, st>>>(offsets, keys, chunks, partials, q.own, buckets,
+                                                                   q.spans);
+    k_fixup_long<<<long_blocks, kLongThreads, 0, st>>>(partials, q.spans, buckets);
+    return cudaGetLastError();
+}
+
 Status scan_u32(Context* ctx, const uint32_t* in, uint32_t* out, uint32_t len, cudaStream_t st) {
     const uint32_t tiles = (len + kScanTile - 1) / kScanTile;
     void* sums;
@@ -839,8 +988,9 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     if (acc_blocks_per_sm < 1) acc_blocks_per_sm = 1;
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
+    const uint32_t quad_blocks = accumulate_quad_blocks(ctx, entries_cap);
 
-    void *counts, *sorted, *partials, *owner, *arena, *wsum;
+    void *counts, *sorted, *partials, *queue, *arena, *wsum;
     void *offsets[kMaxMsmParts] = {}, *buckets[kMaxMsmParts] = {};
     static const char* const kOffsetNames[kMaxMsmParts] = {"msm_offsets", "msm_offsets2", "msm_offsets3",
                                                             "msm_offsets4"};
@@ -855,10 +1005,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     void* digits;
     MZK_TRY(ctx->ensure("msm_digits", entries_cap * 4, &digits));
     MZK_TRY(ctx->ensure("msm_partials", (size_t)acc_threads * 2 * sizeof(Xyzz), &partials));
-    MZK_TRY(ctx->ensure("msm_owner", (size_t)acc_threads * 4, &owner));
-    void *long_count, *long_list;
-    MZK_TRY(ctx->ensure("msm_long_count", 64, &long_count));
-    MZK_TRY(ctx->ensure("msm_long_list", (size_t)acc_threads * sizeof(uint2), &long_list));
+    MZK_TRY(ctx->ensure("msm_queue", queue_bytes(acc_threads), &queue));
     std::vector<Window> wins;
     append_windows(sh, 0, sh.windows, wins);
     const ReducePlan plan = plan_reduce(wins, reduce_group_log(sh.keys, (uint32_t)n_parts));
@@ -900,28 +1047,22 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         MZK_TRY(scan_u32(ctx, (const uint32_t*)counts, off + 1, sh.keys + 1, st));
         MZK_TRY(ctx->phase_end(st));
         MZK_TRY(ctx->phase_begin(PH_SCATTER, st));
-        for (int w = 0; w < sh.windows; w++) {
-            k_scatter_window<<<pt_blocks, pt_threads, 0, st>>>((const uint32_t*)digits + (size_t)w * np, np,
-                                                               off + 1, (uint32_t*)sorted);
+        const uint32_t together = scatter_together((size_t)sh.windows, np);
+        for (uint32_t w = 0; w < (uint32_t)sh.windows; w += together) {
+            const dim3 grid(pt_blocks, std::min(together, (uint32_t)sh.windows - w));
+            k_scatter_window<<<grid, pt_threads, 0, st>>>((const uint32_t*)digits, np, w, off + 1, (uint32_t*)sorted);
             MZK_LAUNCH_CHECK(ctx);
         }
         MZK_TRY(ctx->phase_end(st));
         if (part.bases_ready) MZK_CUDA_CHECK(cudaStreamWaitEvent(st, part.bases_ready, 0));
         MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
-        k_accumulate<<<acc_blocks, kAccThreads, 0, st>>>(ba + part.begin, (const uint32_t*)sorted, off, sh.keys,
-                                                        (Xyzz*)buckets[p], (Xyzz*)partials, (int*)owner);
-        MZK_LAUNCH_CHECK(ctx);
+        MZK_CUDA_CHECK(launch_accumulate(ba + part.begin, (const uint32_t*)sorted, off, sh.keys, (Xyzz*)buckets[p],
+                                         (Xyzz*)partials, queue, acc_blocks, quad_blocks, st));
         MZK_TRY(ctx->phase_end(st));
         MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
-        MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-        k_fixup<<<acc_blocks * 4, kReduceThreads, 0, st>>>(off, sh.keys, acc_threads, (const Xyzz*)partials,
-                                                          (const int*)owner, (Xyzz*)buckets[p],
-                                                          (uint32_t*)long_count, (uint2*)long_list);
-        MZK_LAUNCH_CHECK(ctx);
-        k_fixup_long<<<ctx->num_sms * 2, kLongThreads, 0, st>>>(
-            (const int*)owner, (const Xyzz*)partials, (const uint32_t*)long_count, (const uint2*)long_list,
-            (Xyzz*)buckets[p]);
-        MZK_LAUNCH_CHECK(ctx);
+        MZK_CUDA_CHECK(launch_fixup(off, sh.keys, (Xyzz*)buckets[p], (const Xyzz*)partials, queue, acc_blocks,
+                                    quad_blocks, (uint32_t)ctx->num_sms * 2, st));
+        ctx->launches += 3;
         MZK_TRY(ctx->phase_end(st));
         MZK_CUDA_CHECK(cudaMemcpyAsync(host_entries + p, off + sh.keys, 4, cudaMemcpyDeviceToHost, st));
     }
@@ -1020,10 +1161,12 @@ __global__ void k_digits_batch(const BatchItemDev* __restrict__ items, uint32_t 
 // The batch scatter of window w of every item from the stored digits: the
 // entries land in the items' window-w slices (4 bytes per point of the batch),
 // which stay in L2 while the window is scattered.
-// row_off: w x the table stride (fixed items read window w from table row w)
-__global__ void k_scatter_window_batch(const uint32_t* __restrict__ digits_w, const BatchItemDev* __restrict__ items,
-                                       uint32_t n_items, uint32_t total_points, uint32_t row_off,
+// table_stride: points per table row (fixed items read window w from row w)
+__global__ void k_scatter_window_batch(const uint32_t* __restrict__ digits, const BatchItemDev* __restrict__ items,
+                                       uint32_t n_items, uint32_t total_points, uint32_t w0, uint32_t table_stride,
                                        uint32_t* __restrict__ cursor, uint32_t* __restrict__ sorted) {
+    const uint32_t w = w0 + blockIdx.y, row_off = w * table_stride;
+    const uint32_t* __restrict__ digits_w = digits + (size_t)w * total_points;
     const uint32_t stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -1133,10 +1276,10 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     if (acc_blocks_per_sm < 1) acc_blocks_per_sm = 1;
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
+    const uint32_t quad_blocks = accumulate_quad_blocks(ctx, entries);
     const size_t n_wins = hw.size();
     const ReducePlan plan = plan_reduce(hw, reduce_group_log(keys, 1));
-    void *d_items, *d_tab, *counts, *offsets, *sorted, *buckets, *partials, *owner, *long_count, *long_list, *arena,
-        *wsum;
+    void *d_items, *d_tab, *counts, *offsets, *sorted, *buckets, *partials, *queue, *arena, *wsum;
     MZK_TRY(ctx->ensure("batch_items", hi.size() * sizeof(BatchItemDev), &d_items));
     MZK_TRY(ctx->ensure("batch_wins", plan.table_bytes(), &d_tab));
     MZK_TRY(ctx->ensure("msm_counts", (keys + 1) * 4, &counts));
@@ -1146,9 +1289,7 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     MZK_TRY(ctx->ensure("msm_digits", (size_t)max_windows * points * 4, &digits));
     MZK_TRY(ctx->ensure("msm_buckets", keys * sizeof(Xyzz), &buckets));
     MZK_TRY(ctx->ensure("msm_partials", (size_t)acc_threads * 2 * sizeof(Xyzz), &partials));
-    MZK_TRY(ctx->ensure("msm_owner", (size_t)acc_threads * 4, &owner));
-    MZK_TRY(ctx->ensure("msm_long_count", 64, &long_count));
-    MZK_TRY(ctx->ensure("msm_long_list", (size_t)acc_threads * sizeof(uint2), &long_list));
+    MZK_TRY(ctx->ensure("msm_queue", queue_bytes(acc_threads), &queue));
     MZK_TRY(ctx->ensure("msm_arena", plan.arena * sizeof(Xyzz), &arena));
     MZK_TRY(ctx->ensure("msm_wsum", n_wins * sizeof(Xyzz), &wsum));
     // pinned staging: window sums (read back), then the item table and the reduction's tables
@@ -1178,31 +1319,25 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     MZK_TRY(scan_u32(ctx, (const uint32_t*)counts, (uint32_t*)offsets + 1, (uint32_t)keys + 1, st));
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_SCATTER, st));
-    for (int w = 0; w < max_windows; w++) {
-        const uint32_t row_off = table ? (uint32_t)((uint64_t)w * table->stride) : 0u;
-        k_scatter_window_batch<<<pt_blocks, pt_threads, 0, st>>>((const uint32_t*)digits + (size_t)w * points,
-                                                                 (const BatchItemDev*)d_items, n_items,
-                                                                 (uint32_t)points, row_off,
-                                                                 (uint32_t*)offsets + 1, (uint32_t*)sorted);
+    const uint32_t together = scatter_together((size_t)max_windows, points);
+    for (uint32_t w = 0; w < (uint32_t)max_windows; w += together) {
+        const dim3 grid(pt_blocks, std::min(together, (uint32_t)max_windows - w));
+        k_scatter_window_batch<<<grid, pt_threads, 0, st>>>((const uint32_t*)digits, (const BatchItemDev*)d_items,
+                                                            n_items, (uint32_t)points, w,
+                                                            table ? (uint32_t)table->stride : 0u,
+                                                            (uint32_t*)offsets + 1, (uint32_t*)sorted);
         MZK_LAUNCH_CHECK(ctx);
     }
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
-    k_accumulate<<<acc_blocks, kAccThreads, 0, st>>>(static_cast<const Affine*>(d_bases), (const uint32_t*)sorted,
-                                                    (const uint32_t*)offsets, (uint32_t)keys, (Xyzz*)buckets,
-                                                    (Xyzz*)partials, (int*)owner);
-    MZK_LAUNCH_CHECK(ctx);
+    MZK_CUDA_CHECK(launch_accumulate(static_cast<const Affine*>(d_bases), (const uint32_t*)sorted,
+                                     (const uint32_t*)offsets, (uint32_t)keys, (Xyzz*)buckets, (Xyzz*)partials, queue,
+                                     acc_blocks, quad_blocks, st));
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
-    MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-    k_fixup<<<acc_blocks * 4, kReduceThreads, 0, st>>>((const uint32_t*)offsets, (uint32_t)keys, acc_threads,
-                                                      (const Xyzz*)partials, (const int*)owner, (Xyzz*)buckets,
-                                                      (uint32_t*)long_count, (uint2*)long_list);
-    MZK_LAUNCH_CHECK(ctx);
-    k_fixup_long<<<ctx->num_sms * 2, kLongThreads, 0, st>>>(
-        (const int*)owner, (const Xyzz*)partials, (const uint32_t*)long_count, (const uint2*)long_list,
-        (Xyzz*)buckets);
-    MZK_LAUNCH_CHECK(ctx);
+    MZK_CUDA_CHECK(launch_fixup((const uint32_t*)offsets, (uint32_t)keys, (Xyzz*)buckets, (const Xyzz*)partials,
+                                queue, acc_blocks, quad_blocks, (uint32_t)ctx->num_sms * 2, st));
+    ctx->launches += 3;
     MZK_TRY(ctx->phase_end(st));
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
     const BucketSets sets{{(const Xyzz*)buckets}, {(const uint32_t*)offsets}, 1};
@@ -1280,8 +1415,8 @@ constexpr size_t kNaOffsetsOff = kNaCountsOff + align256((kNaKeys + 1) * 4);
 constexpr size_t kNaSortedOff = kNaOffsetsOff + align256((kNaKeys + 2) * 4);
 constexpr size_t kNaBucketsOff = kNaSortedOff + align256(kNaMaxWindows * kNoAllocMaxN * 4);
 constexpr size_t kNaPartialsOff = kNaBucketsOff + align256(kNaKeys * sizeof(Xyzz));
-constexpr size_t kNaOwnerOff = kNaPartialsOff + align256(kNaAccThreads * 2 * sizeof(Xyzz));
-constexpr size_t kNaArenaOff = kNaOwnerOff + align256(kNaAccThreads * 4);
+constexpr size_t kNaQueueOff = kNaPartialsOff + align256(kNaAccThreads * 2 * sizeof(Xyzz));
+constexpr size_t kNaArenaOff = kNaQueueOff + align256(queue_bytes(kNaAccThreads));
 // the reduction tree's values over the widest key count: a node of 64 buckets
 // leaves 7 values, and the one or two launches above it far fewer
 constexpr size_t kNaArenaPoints = kNaKeys / 64 * 7 + kNaMaxWindows * 32;
@@ -1289,8 +1424,7 @@ constexpr size_t kNaTabBytes = kNaMaxWindows * (4 * sizeof(TreeWin) + sizeof(Fin
 constexpr size_t kNaWsumOff = kNaArenaOff + align256(kNaArenaPoints * sizeof(Xyzz));
 constexpr size_t kNaScanOff = kNaWsumOff + align256(kNaMaxWindows * sizeof(Xyzz));
 constexpr size_t kNaWinsOff = kNaScanOff + align256(64 * 4);
-constexpr size_t kNaLongOff = kNaWinsOff + align256(kNaTabBytes);
-constexpr size_t kNaBytes = kNaLongOff + align256(16 + kNaAccThreads * sizeof(uint2));
+constexpr size_t kNaBytes = kNaWinsOff + align256(kNaTabBytes);
 
 // The scratch itself.  Host code must not use this name as a device address:
 // on the host it is only a stand-in, so kernels get the pointer obtained from
@@ -1364,7 +1498,7 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
     uint32_t* sorted = reinterpret_cast<uint32_t*>(base + kNaSortedOff);
     Xyzz* buckets = reinterpret_cast<Xyzz*>(base + kNaBucketsOff);
     Xyzz* partials = reinterpret_cast<Xyzz*>(base + kNaPartialsOff);
-    int* owner = reinterpret_cast<int*>(base + kNaOwnerOff);
+    void* queue = base + kNaQueueOff;
     Xyzz* arena = reinterpret_cast<Xyzz*>(base + kNaArenaOff);
     Xyzz* wsum = reinterpret_cast<Xyzz*>(base + kNaWsumOff);
     uint32_t* scan_sums = reinterpret_cast<uint32_t*>(base + kNaScanOff);
@@ -1382,16 +1516,9 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
     MZK_TRY(scan_u32_noalloc(counts, offsets + 1, sh.keys + 1, scan_sums, st));
     k_scatter<<<pt_blocks, pt_threads, 0, st>>>(sc, n, sh.c, sh.windows, sh.nb, offsets + 1, sorted);
     MZK_CUDA_CHECK(cudaGetLastError());
-    k_accumulate<<<kNoAllocAccBlocks, kAccThreads, 0, st>>>(ba, sorted, offsets, sh.keys, buckets, partials, owner);
-    MZK_CUDA_CHECK(cudaGetLastError());
-    uint32_t* long_count = reinterpret_cast<uint32_t*>(base + kNaLongOff);
-    uint2* long_list = reinterpret_cast<uint2*>(base + kNaLongOff + 16);
-    MZK_CUDA_CHECK(cudaMemsetAsync(long_count, 0, 4, st));
-    k_fixup<<<kNoAllocAccBlocks * 4, kReduceThreads, 0, st>>>(offsets, sh.keys, (uint32_t)kNaAccThreads, partials,
-                                                             owner, buckets, long_count, long_list);
-    MZK_CUDA_CHECK(cudaGetLastError());
-    k_fixup_long<<<kNoAllocAccBlocks, kLongThreads, 0, st>>>(owner, partials, long_count, long_list, buckets);
-    MZK_CUDA_CHECK(cudaGetLastError());
+    // (by lanes: the fixed grid of 64 blocks holds 2048 quads only)
+    MZK_CUDA_CHECK(launch_accumulate(ba, sorted, offsets, sh.keys, buckets, partials, queue, kNoAllocAccBlocks, 0, st));
+    MZK_CUDA_CHECK(launch_fixup(offsets, sh.keys, buckets, partials, queue, kNoAllocAccBlocks, 0, kNoAllocAccBlocks, st));
     // the reduction's tables (a copy from pageable memory is staged before the call returns)
     std::vector<Window> wins;
     append_windows(sh, 0, sh.windows, wins);

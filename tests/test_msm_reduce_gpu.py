@@ -70,3 +70,20 @@ def test_reduction_matches_the_plain_sum(ctx, c, kind):
     finally:
         ctx.set_msm_window(0)
     assert np.array_equal(mzk.affine(got), O.msm_naive(s, b))
+
+
+# 29 windows of width 9: 149988 and 150017 digits, either side of the line between quads and lanes per chunk
+@pytest.mark.parametrize("n", [5172, 5173])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_accumulation_by_quads_and_by_lanes(ctx, n, sparse):
+    s, b = O.rand_fr(17, n), O.gen_bases(19, n)
+    if sparse:  # heavy buckets and an identity base
+        s[:n // 2] = O.fr_const(0)
+        s[n // 2:2 * n // 3] = 0
+        b[5] = 0
+    ctx.set_msm_window(9)
+    try:
+        got = ctx.msm_best(s, b)
+    finally:
+        ctx.set_msm_window(0)
+    assert np.array_equal(mzk.affine(got), O.msm_best(s, b))
