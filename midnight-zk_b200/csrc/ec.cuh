@@ -9,6 +9,7 @@
 // of blst_p1_affine used by the reference (curves/src/bls12_381/g1.rs:761-763).
 #pragma once
 #include "field.cuh"
+#include "inv.cuh"
 
 namespace mzk {
 
@@ -188,7 +189,7 @@ __device__ __forceinline__ Affine xyzz_to_affine(const Xyzz& p) {
         return a;
     }
     // 1/ZZZ, then 1/ZZ = (ZZ/ZZZ)^2
-    Fp t = fp_inv(p.zzz);
+    Fp t = fp_invert(p.zzz);
     Fp zi = fp_mul(p.zz, t);
     Fp zi2 = fp_sqr(zi);
     a.x = fp_canonical(fp_mul(p.x, zi2));

@@ -22,8 +22,9 @@
 
 #include "../../include/mzk.h"
 #include "field.cuh"
-#include "host_ec.hpp"
 #include "grand.hpp"
+#include "host_ec.hpp"
+#include "inv.cuh"
 #include "ntt.hpp"
 #include "runtime.hpp"
 
@@ -44,20 +45,6 @@ __device__ __forceinline__ bool fr_is_zero(const Fr& a) {
 #pragma unroll
     for (int j = 0; j < 8; j++) acc |= a.l[j];
     return acc == 0;
-}
-
-// 1/a for a non-zero a (zero gives zero): the binary extended Euclidean
-// algorithm (inv_binary_raw) on the stored Montgomery limbs A = a R yields
-// A^-1 = a^-1 R^-1, and one Montgomery product with R^3 gives a^-1 R, the
-// Montgomery form of 1/a.  A block's single inversion is a serial chain on
-// one thread, and this finishes it several times sooner than a Fermat
-// power.  Variable time in the value.
-__device__ __noinline__ Fr fr_inv(const Fr& a) {
-    Fr x, r2;
-    if (!inv_binary_raw<8>(x.l, a.l, FrMod())) return fr_zero();
-#pragma unroll
-    for (int j = 0; j < 8; j++) r2.l[j] = FrP::r2(j);
-    return fr_mul(x, fr_mul(r2, r2));  // x R^3 R^-1 = a^-1 R
 }
 
 Fr to_dev(const host::Fr4& h) {
@@ -128,10 +115,11 @@ __device__ Fr block_exclusive_suffix_product(Fr v, Fr* sm) {
 // threads' products by a prefix and a suffix scan in shared memory, and the
 // inverse of the block's total gives every thread the inverse of its product
 // (prefix x suffix x 1/total); the backward pass then inverts each element.
-// The inverse of the total is one Fermat inversion in the block when the
-// blocks fit one wave on the GPU; otherwise the totals are batch-inverted
-// first (k_invert_totals, then this function on the totals), since a serial
-// inversion per block would leave the SMs idle wave after wave.
+// The inverse of the total is one inversion by one thread of the block (17.6
+// us; by binary extended Euclid it took 54) when the blocks fit one wave on the
+// GPU; otherwise the totals are batch-inverted first (k_invert_totals, then
+// this function on the totals), since a serial inversion per block would leave
+// the SMs idle wave after wave.
 constexpr int kInvPerThread = 4;
 
 template <int C>
@@ -173,7 +161,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_invert(Fr* __restrict__ a, u
     Fr total;
     const Fr below = block_exclusive<true>(acc, sm, &total);
     const Fr above = block_exclusive_suffix_product(acc, sm);
-    if (threadIdx.x == 0) total_inv = kGivenInverse ? tot_inv[blockIdx.x] : fr_inv(total);
+    if (threadIdx.x == 0) total_inv = kGivenInverse ? tot_inv[blockIdx.x] : fr_invert(total);
     __syncthreads();
     Fr inv = fr_mul(fr_mul(total_inv, below), above);  // 1 / acc
 #pragma unroll

@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(128) k_probe_batch_affine(uint32_t seed, uint3
     if (acc == 0x12345678u) sink[0] = acc;
 }
 
-// Self-check of the binary inversion: a^-1 a = 1 for every input (the
-// Montgomery one), and the inverse equals the Fermat power's.
+// Self-check of the binary inversion and of the one by division steps: a^-1 a
+// = 1 for every input (the Montgomery one), and both equal the Fermat power.
 __global__ void k_check_fp_inv(const Fp* __restrict__ in, size_t n, unsigned long long* __restrict__ mismatches) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -212,9 +212,10 @@ __global__ void k_check_fp_inv(const Fp* __restrict__ in, size_t n, unsigned lon
         const Fp inv = fp_canonical(fp_mul(x, fp_mul(r2, r2)));
         const Fp ferm = fp_canonical(fp_inv(a));
         const Fp one = fp_canonical(fp_mul(inv, a));
+        const Fp steps = fp_invert(in[i]);  // as given: lazily reduced values too
         uint32_t diff = 0;
 #pragma unroll
-        for (int j = 0; j < 12; j++) diff |= (inv.l[j] ^ ferm.l[j]) | (one.l[j] ^ FpP::one(j));
+        for (int j = 0; j < 12; j++) diff |= (inv.l[j] ^ ferm.l[j]) | (steps.l[j] ^ ferm.l[j]) | (one.l[j] ^ FpP::one(j));
         if (diff) atomicAdd(mismatches, 1ull);
     }
 }
