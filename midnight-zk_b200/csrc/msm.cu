@@ -254,6 +254,9 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
     return prefix + x - v;
 }
 
+// kHalves: `in` is an offset table of len - 1 buckets and the scanned values
+// are the buckets' sizes after one round of pair sums (half, rounded up), then 0
+template <bool kHalves>
 __global__ void k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t len,
                              uint32_t* __restrict__ tile_sums) {
     __shared__ uint32_t sw[32];
@@ -261,7 +264,8 @@ __global__ void k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restri
     uint32_t v[kScanItems], sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        v[k] = base + k < len ? in[base + k] : 0;
+        if (kHalves) v[k] = base + k + 1 < len ? (in[base + k + 1] - in[base + k] + 1) >> 1 : 0;
+        else v[k] = base + k < len ? in[base + k] : 0;
         sum += v[k];
     }
     uint32_t total;
@@ -354,6 +358,9 @@ __device__ __forceinline__ void flush_bucket(const Xyzz& acc, uint32_t k, uint32
     }
 }
 
+// kGather: entry j is the point sorted[j] (index | sign); otherwise point j of
+// `bases` itself (the pair sums of k_pair_sums).
+template <bool kGather>
 __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __restrict__ bases,
                                                             const uint32_t* __restrict__ sorted,
                                                             const uint32_t* __restrict__ offsets, uint32_t keys,
@@ -374,9 +381,9 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
     xyzz_set_inf(acc);
     // the next entry's base is loaded one iteration ahead, and the entry after
     // it (its index) two ahead, to hide the gather latency
-    uint32_t ent = __ldg(sorted + s);
-    uint32_t ent2 = s + 1 < e ? __ldg(sorted + s + 1) : 0u;
-    Affine nxt = load_affine(bases, ent & 0x7fffffffu);
+    uint32_t ent = kGather ? __ldg(sorted + s) : s;
+    uint32_t ent2 = s + 1 < e ? (kGather ? __ldg(sorted + s + 1) : s + 1) : 0u;
+    Affine nxt = load_affine(bases, kGather ? ent & 0x7fffffffu : ent);
     for (uint32_t j = s; j < e; j++) {
         if (j == seg_hi) {
             flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, own);
@@ -395,11 +402,11 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
         const uint32_t cur = ent;
         if (j + 1 < e) {
             ent = ent2;
-            nxt = load_affine(bases, ent & 0x7fffffffu);
-            if (j + 2 < e) ent2 = __ldg(sorted + j + 2);
+            nxt = load_affine(bases, kGather ? ent & 0x7fffffffu : ent);
+            if (j + 2 < e) ent2 = kGather ? __ldg(sorted + j + 2) : j + 2;
         }
         if (aff_is_inf(p)) continue;
-        p.y = fp_select((cur >> 31) != 0, fp_neg(p.y), p.y);
+        if (kGather) p.y = fp_select((cur >> 31) != 0, fp_neg(p.y), p.y);
         if (xyzz_is_inf(acc)) {
             acc.x = p.x;
             acc.y = p.y;
@@ -410,6 +417,216 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
         }
     }
     flush_bucket(acc, k, seg_lo, seg_hi, s, e, t, buckets, partials, own);
+}
+
+// ---- pair sums ----
+//
+// One round replaces the points of every bucket by the sums of neighbours, in
+// affine coordinates, so that half as many are left for k_accumulate.  An
+// affine addition takes 5 products, a square and an inversion; each thread
+// shares one inversion among its B additions by Montgomery's trick (3 of the
+// products).  With ~40 products' worth of time for the inversion
+// (inv_divsteps) an addition costs ~7 products against the 10 of a mixed XYZZ
+// addition, at the price of writing the sums (96 bytes each) and reading them
+// again.  The multiply pipe is 70-72 % busy (88 % in k_accumulate): the rest
+// are waits for loads that one sum's lead does not cover and, with two warps
+// per scheduler, the latency of the products themselves.  1000003 points: 8.4 M
+// + 4.2 M + 2.1 M sums take 2.33 + 1.24 + 0.64 ms and leave 0.83 ms of mixed
+// additions, 5.8 ms without.  A third warp per scheduler spills (168
+// registers) and is slower (7.34 ms per call against 6.66), as are 48 sums per
+// inversion.
+//
+// A thread takes a run of consecutive sums: forward it multiplies up the
+// denominators and keeps the partial products, then inverts, then backward it
+// forms the sums.  A bucket's odd last point is copied.
+__device__ __forceinline__ Fp load_fp(const Fp* p) {
+    const uint4* s = reinterpret_cast<const uint4*>(p);
+    Fp r;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint4 v = __ldg(s + k);
+        r.l[4 * k] = v.x;
+        r.l[4 * k + 1] = v.y;
+        r.l[4 * k + 2] = v.z;
+        r.l[4 * k + 3] = v.w;
+    }
+    return r;
+}
+__device__ __forceinline__ void store_affine(Affine* dst, const Affine& a) {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    const uint32_t* s = reinterpret_cast<const uint32_t*>(&a);
+#pragma unroll
+    for (int k = 0; k < 6; k++) d[k] = make_uint4(s[4 * k], s[4 * k + 1], s[4 * k + 2], s[4 * k + 3]);
+}
+
+// The cases of a + b whose sum is not the chord's: what to do, the denominator
+// that enters the shared inversion and the slope's numerator.  By value, so
+// that the loop's points stay in registers.
+enum PairKind : int { kPairAdd, kPairFirst, kPairSecond, kPairDouble, kPairInfinity };
+struct PairCase {
+    Fp den, num;
+    int kind;
+};
+static __device__ __noinline__ PairCase pair_case(const Affine a, const Affine b) {
+    PairCase c;
+    c.den = fp_sub(b.x, a.x);
+    c.num = fp_sub(b.y, a.y);
+    if (aff_is_inf(a)) {
+        c.kind = kPairSecond;
+    } else if (aff_is_inf(b)) {
+        c.kind = kPairFirst;
+    } else if (!fp_is_zero(c.den)) {
+        c.kind = kPairAdd;
+    } else if (!fp_is_zero(c.num)) {
+        c.kind = kPairInfinity;
+    } else {
+        const Fp xx = fp_mul(a.x, a.x);
+        c.kind = kPairDouble;
+        c.num = fp_add(fp_dbl(xx), xx);
+        c.den = fp_dbl(a.y);  // not zero: the curve has no point of order 2
+    }
+    return c;
+}
+
+constexpr int kPairThreads = 128;
+constexpr int kPairBatch = 64;  // sums that share an inversion
+
+// Sum j of bucket k: points off_in[k] + 2 (j - off_out[k]) and the next, if
+// that is below off_in[k + 1].  kGather: point i is src[sorted[i]] with the
+// entry's sign, otherwise src[i].
+template <int B, bool kGather>
+__global__ void __launch_bounds__(kPairThreads, 2) k_pair_sums(const Affine* __restrict__ src,
+                                                               const uint32_t* __restrict__ sorted,
+                                                               const uint32_t* __restrict__ off_in,
+                                                               const uint32_t* __restrict__ off_out, uint32_t keys,
+                                                               Affine* __restrict__ out) {
+    static_assert(B <= 64, "a bit per sum");
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t s, e;
+    chunk_range(off_out[keys], t, gridDim.x * blockDim.x, s, e);
+    if (s >= e) return;
+    // the point of an entry: index | sign << 31 when gathering, else the index
+    auto point = [&](uint32_t ent) { return load_affine(src, kGather ? ent & 0x7fffffffu : ent); };
+    auto signed_point = [&](Affine a, uint32_t ent) {
+        if (kGather) a.y = fp_select((ent >> 31) != 0, fp_neg(a.y), a.y);
+        return a;
+    };
+    auto point_x = [&](uint32_t ent) { return load_fp(&src[kGather ? ent & 0x7fffffffu : ent].x); };
+    uint32_t k = find_key(off_out, keys, s);
+    uint32_t lo = off_out[k], hi = off_out[k + 1], in_lo = off_in[k], in_hi = off_in[k + 1];
+    const uint32_t rounds = (e - s + B - 1) / B, per = (e - s + rounds - 1) / rounds;
+    Fp prefix[B];
+    uint32_t ent1[B], ent2[B];
+    for (uint32_t j0 = s; j0 < e; j0 += per) {
+        const int n = (int)min(per, e - j0);
+        uint64_t pairs = 0, plain = 0;  // sum i adds two points; by the chord of two finite points
+        for (int i = 0; i < n; i++) {
+            const uint32_t j = j0 + (uint32_t)i;
+            while (j >= hi) {
+                k++;
+                lo = hi;
+                hi = off_out[k + 1];
+                in_lo = off_in[k];
+                in_hi = off_in[k + 1];
+            }
+            const uint32_t p = in_lo + 2 * (j - lo);
+            const bool two = p + 1 < in_hi;
+            ent1[i] = kGather ? __ldg(sorted + p) : p;
+            ent2[i] = kGather ? (two ? __ldg(sorted + p + 1) : 0u) : p + 1;
+            if (two) pairs |= 1ull << i;
+        }
+        // forward: the x of the next sum's points are loaded one sum ahead and
+        // its entries two, so that no address waits on a load
+        uint32_t c1 = ent1[0], c2 = ent2[0], e1 = 0, e2 = 0;
+        Fp acc = fp_one(), n1 = fp_zero(), n2 = fp_zero();
+        if (pairs & 1ull) {
+            n1 = point_x(c1);
+            n2 = point_x(c2);
+        }
+        if (n > 1) {
+            e1 = ent1[1];
+            e2 = ent2[1];
+        }
+        for (int i = 0; i < n; i++) {
+            const Fp x1 = n1, x2 = n2;
+            const uint32_t p1 = c1, p2 = c2;
+            c1 = e1;
+            c2 = e2;
+            if (i + 2 < n) {
+                e1 = ent1[i + 2];
+                e2 = ent2[i + 2];
+            }
+            if (i + 1 < n && ((pairs >> (i + 1)) & 1ull)) {
+                n1 = point_x(c1);
+                n2 = point_x(c2);
+            }
+            if (!((pairs >> i) & 1ull)) continue;
+            Fp d = fp_sub(x2, x1);
+            if (fp_is_zero(d) || fp_is_zero_raw(x1) || fp_is_zero_raw(x2)) {  // rare, infinity among them
+                const PairCase c = pair_case(signed_point(point(p1), p1), signed_point(point(p2), p2));
+                if (c.kind == kPairFirst || c.kind == kPairSecond || c.kind == kPairInfinity) continue;
+                d = c.den;
+            } else {
+                plain |= 1ull << i;
+            }
+            prefix[i] = acc;
+            acc = fp_mul(acc, d);
+        }
+        Fp inv = fp_invert(acc);
+        // backward: points and partial product one sum ahead, entries two
+        c1 = ent1[n - 1];
+        c2 = ent2[n - 1];
+        if (n > 1) {
+            e1 = ent1[n - 2];
+            e2 = ent2[n - 2];
+        }
+        Affine na = point(c1), nb = na;
+        Fp npre = prefix[n - 1];
+        if ((pairs >> (n - 1)) & 1ull) nb = point(c2);
+        for (int i = n - 1; i >= 0; i--) {
+            Affine a = signed_point(na, c1);
+            const Affine b = signed_point(nb, c2);
+            const Fp pre = npre;
+            c1 = e1;
+            c2 = e2;
+            if (i > 1) {
+                e1 = ent1[i - 2];
+                e2 = ent2[i - 2];
+            }
+            if (i > 0) {
+                na = point(c1);
+                if ((pairs >> (i - 1)) & 1ull) {
+                    nb = point(c2);
+                    npre = prefix[i - 1];
+                }
+            }
+            if ((pairs >> i) & 1ull) {
+                Fp d = fp_sub(b.x, a.x), num = fp_sub(b.y, a.y);
+                int kind = kPairAdd;
+                if (!((plain >> i) & 1ull)) {
+                    const PairCase c = pair_case(a, b);
+                    kind = c.kind;
+                    d = c.den;
+                    num = c.num;
+                }
+                if (kind == kPairSecond) {
+                    a = b;
+                } else if (kind == kPairInfinity) {
+                    a.x = fp_zero();
+                    a.y = fp_zero();
+                } else if (kind != kPairFirst) {
+                    Fp di, next;
+                    fp_mul2(di, inv, pre, next, inv, d);
+                    inv = next;
+                    const Fp lam = fp_mul(num, di);
+                    const Fp x3 = fp_sub(fp_sub(fp_sqr(lam), a.x), b.x);
+                    a.y = fp_sub(fp_mul(lam, fp_sub(a.x, x3)), a.y);
+                    a.x = x3;
+                }
+            }
+            store_affine(&out[j0 + (uint32_t)i], a);
+        }
+    }
 }
 
 // The same walk with one quad of lanes per chunk, for inputs too small to fill
@@ -885,42 +1102,158 @@ Queues queues_at(void* p, size_t chunks) {
     return {{counts, reinterpret_cast<uint2*>(spans + chunks)}, {counts + 1, spans}};
 }
 
-// The bucket accumulation, by quads (quad_blocks > 0) or by lanes, and the
-// sums of the buckets that its chunks cut.  `queue` holds queue_bytes of the
-// lanes' grid, which is the larger one.  Returns the launch error, if any.
-cudaError_t launch_accumulate(const Affine* bases, const uint32_t* sorted, const uint32_t* offsets, uint32_t keys,
-                              Xyzz* buckets, Xyzz* partials, void* queue, uint32_t acc_blocks, uint32_t quad_blocks,
-                              cudaStream_t st) {
-    const Queues q = queues_at(queue, (size_t)acc_blocks * kAccThreads);
-    const cudaError_t e = cudaMemsetAsync(queue, 0, 16, st);
-    if (e != cudaSuccess) return e;
-    if (quad_blocks)
-        k_accumulate_quads<<<quad_blocks, kAccThreads, 0, st>>>(bases, sorted, offsets, keys, buckets, partials, q.own);
-    else
-        k_accumulate<<<acc_blocks, kAccThreads, 0, st>>>(bases, sorted, offsets, keys, buckets, partials, q.own);
-    return cudaGetLastError();
-}
-cudaError_t launch_fixup(const uint32_t* offsets, uint32_t keys, Xyzz* buckets, const Xyzz* partials, void* queue,
-                         uint32_t acc_blocks, uint32_t quad_blocks, uint32_t long_blocks, cudaStream_t st) {
-    const Queues q = queues_at(queue, (size_t)acc_blocks * kAccThreads);
-    const uint32_t chunks = quad_blocks ? quad_blocks * (kAccThreads / 4) : acc_blocks * kAccThreads;
-    k_fixup<<<chunks * 4 / kReduceThreads, kReduceThreads, 0, st>>>(offsets, keys, chunks, partials, q.own, buckets,
-                                                                   q.spans);
-    k_fixup_long<<<long_blocks, kLongThreads, 0, st>>>(partials, q.spans, buckets);
-    return cudaGetLastError();
-}
-
+template <bool kHalves = false>
 Status scan_u32(Context* ctx, const uint32_t* in, uint32_t* out, uint32_t len, cudaStream_t st) {
     const uint32_t tiles = (len + kScanTile - 1) / kScanTile;
     void* sums;
     MZK_TRY(ctx->ensure("scan_sums", (size_t)tiles * 4 + 64, &sums));
-    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(in, out, len, (uint32_t*)sums);
+    k_scan_tiles<kHalves><<<tiles, kScanThreads, 0, st>>>(in, out, len, (uint32_t*)sums);
     MZK_LAUNCH_CHECK(ctx);
     k_scan_sums<<<1, kScanThreads, 0, st>>>((uint32_t*)sums, tiles);
     MZK_LAUNCH_CHECK(ctx);
     k_scan_add<<<tiles, kScanThreads, 0, st>>>(out, len, (const uint32_t*)sums);
     MZK_LAUNCH_CHECK(ctx);
     return OK;
+}
+
+// What the accumulation of one sorted entry array needs
+struct Accumulation {
+    const Affine* bases;
+    const uint32_t* sorted;
+    const uint32_t* offsets;  // keys + 2
+    uint32_t keys;
+    Xyzz* buckets;
+    Xyzz* partials;
+    void* queue;           // queue_bytes of the lanes' grid, which is the larger one
+    uint32_t acc_blocks;   // lanes' grid
+    uint32_t quad_blocks;  // > 0: by quads
+    uint32_t long_blocks;
+};
+
+// The bucket sums by quads or by lanes (gather: see k_accumulate).  Returns
+// the launch error, if any.
+cudaError_t launch_accumulate(const Accumulation& a, bool gather, cudaStream_t st) {
+    const Queues q = queues_at(a.queue, (size_t)a.acc_blocks * kAccThreads);
+    cudaError_t e = cudaMemsetAsync(a.queue, 0, 16, st);
+    if (e != cudaSuccess) return e;
+    if (a.quad_blocks)
+        k_accumulate_quads<<<a.quad_blocks, kAccThreads, 0, st>>>(a.bases, a.sorted, a.offsets, a.keys, a.buckets,
+                                                                  a.partials, q.own);
+    else if (gather)
+        k_accumulate<true><<<a.acc_blocks, kAccThreads, 0, st>>>(a.bases, a.sorted, a.offsets, a.keys, a.buckets,
+                                                                 a.partials, q.own);
+    else
+        k_accumulate<false><<<a.acc_blocks, kAccThreads, 0, st>>>(a.bases, nullptr, a.offsets, a.keys, a.buckets,
+                                                                  a.partials, q.own);
+    return cudaGetLastError();
+}
+
+// The sums of the buckets that the chunks cut.
+cudaError_t launch_fixup(const Accumulation& a, cudaStream_t st) {
+    const Queues q = queues_at(a.queue, (size_t)a.acc_blocks * kAccThreads);
+    const uint32_t chunks = a.quad_blocks ? a.quad_blocks * (kAccThreads / 4) : a.acc_blocks * kAccThreads;
+    k_fixup<<<chunks * 4 / kReduceThreads, kReduceThreads, 0, st>>>(a.offsets, a.keys, chunks, a.partials, q.own,
+                                                                   a.buckets, q.spans);
+    k_fixup_long<<<a.long_blocks, kLongThreads, 0, st>>>(a.partials, q.spans, a.buckets);
+    return cudaGetLastError();
+}
+
+// Consecutive keys and the most entries they can hold
+struct KeyRange {
+    uint32_t key_end;
+    uint64_t entries;
+};
+
+// Rounds of pair sums for `entries` entries over `keys` buckets.  A sum costs
+// less than a mixed addition only while a thread has ~48 to share an inversion
+// (the lanes' grid has 37888 threads), and a round halves buckets of four
+// points or more.  Per call without / with 1 / 2 / 3 rounds: 1000003 points (16.8
+// M entries, 32 per bucket) 7.34 / 6.86 / 6.73 / 6.66 ms, 4000000 points 25.4 /
+// 23.5 / 22.6 / 22.2, 2^24 points 92.0 / 90.0 / 88.0 / 87.4; 262144 points (5 M
+// entries) 2.60 / 2.59 / 2.59 / 2.62.
+constexpr uint64_t kPairsPerRound = 48 * 37888;
+constexpr int kPairRounds = 3;
+
+int pair_rounds(uint64_t entries, uint64_t keys) {
+    int r = 0;
+    while (r < kPairRounds && (entries >> (r + 1)) >= kPairsPerRound && (entries >> r) >= 4 * keys) r++;
+    return r;
+}
+
+// The bucket sums of all keys, by rounds of pair sums first where they pay.
+// The sums are formed for a part of the keys at a time (whole ranges, up to
+// kPairEntries entries), so that their arrays stay a few GB at any size.
+// Without memory for them the entries are accumulated as they are.  `entries`
+// is an upper bound (no zero digits); where it may call for rounds the true
+// number, which decides, is read back through `total` (pinned).
+constexpr uint64_t kPairEntries = 1u << 25;
+
+Status accumulate(Context* ctx, const Accumulation& all, const std::vector<KeyRange>& ranges, uint64_t entries,
+                  uint32_t* total, cudaStream_t st) {
+    int rounds = all.quad_blocks ? 0 : pair_rounds(entries, all.keys);
+    if (rounds) {
+        MZK_CUDA_CHECK(cudaMemcpyAsync(total, all.offsets + all.keys, 4, cudaMemcpyDeviceToHost, st));
+        MZK_CUDA_CHECK(cudaStreamSynchronize(st));
+        rounds = pair_rounds(*total, all.keys);
+    }
+    struct Part {
+        uint32_t k0, k1;
+        uint64_t entries;
+    };
+    std::vector<Part> parts;
+    uint64_t most = 0, most_keys = 0;
+    if (rounds) {
+        uint32_t k = 0;
+        for (const KeyRange& r : ranges) {
+            if (parts.empty() || parts.back().entries + r.entries > kPairEntries) parts.push_back({k, k, 0});
+            parts.back().k1 = k = r.key_end;
+            parts.back().entries += r.entries;
+        }
+        for (const Part& p : parts) {
+            most = std::max(most, p.entries);
+            most_keys = std::max<uint64_t>(most_keys, p.k1 - p.k0);
+        }
+    }
+    void *sums[2] = {}, *offs[2] = {};
+    bool paired = rounds > 0;
+    if (paired) {
+        const uint64_t cap0 = (most + most_keys) / 2 + 1, cap1 = (cap0 + most_keys) / 2 + 1;
+        paired = ctx->ensure("msm_sums0", cap0 * sizeof(Affine), &sums[0]) == OK &&
+                 (rounds < 2 || ctx->ensure("msm_sums1", cap1 * sizeof(Affine), &sums[1]) == OK) &&
+                 ctx->ensure("msm_sum_off0", (most_keys + 2) * 4, &offs[0]) == OK &&
+                 (rounds < 2 || ctx->ensure("msm_sum_off1", (most_keys + 2) * 4, &offs[1]) == OK);
+    }
+    MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
+    if (!paired) parts.assign(1, {0, all.keys, entries});
+    int per_sm = 0;
+    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_sums<kPairBatch, true>, kPairThreads, 0));
+    const uint32_t blocks = (uint32_t)ctx->num_sms * (uint32_t)std::max(1, per_sm);
+    for (const Part& p : parts) {
+        Accumulation a = all;
+        a.keys = p.k1 - p.k0;
+        a.buckets = all.buckets + p.k0;
+        a.offsets = all.offsets + p.k0;
+        for (int r = 0; paired && r < rounds; r++) {
+            uint32_t* off = static_cast<uint32_t*>(offs[r & 1]);
+            Affine* out = static_cast<Affine*>(sums[r & 1]);
+            MZK_TRY(scan_u32<true>(ctx, a.offsets, off, a.keys + 1, st));
+            if (r == 0)
+                k_pair_sums<kPairBatch, true><<<blocks, kPairThreads, 0, st>>>(a.bases, a.sorted, a.offsets, off, a.keys, out);
+            else
+                k_pair_sums<kPairBatch, false><<<blocks, kPairThreads, 0, st>>>(a.bases, nullptr, a.offsets, off, a.keys, out);
+            MZK_LAUNCH_CHECK(ctx);
+            a.offsets = off;
+            a.bases = out;
+        }
+        MZK_CUDA_CHECK(launch_accumulate(a, !paired, st));
+        if (&p == &parts.back()) {  // one phase each per call, whatever the parts
+            MZK_TRY(ctx->phase_end(st));
+            MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
+        }
+        MZK_CUDA_CHECK(launch_fixup(a, st));
+        ctx->launches += 3;
+    }
+    return ctx->phase_end(st);
 }
 
 }  // namespace
@@ -984,7 +1317,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
     }
     // accumulate grid: persistent, sized to fill the GPU once
     int acc_blocks_per_sm = 0;
-    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&acc_blocks_per_sm, k_accumulate, kAccThreads, 0));
+    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&acc_blocks_per_sm, k_accumulate<true>, kAccThreads, 0));
     if (acc_blocks_per_sm < 1) acc_blocks_per_sm = 1;
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
@@ -1055,15 +1388,11 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         }
         MZK_TRY(ctx->phase_end(st));
         if (part.bases_ready) MZK_CUDA_CHECK(cudaStreamWaitEvent(st, part.bases_ready, 0));
-        MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
-        MZK_CUDA_CHECK(launch_accumulate(ba + part.begin, (const uint32_t*)sorted, off, sh.keys, (Xyzz*)buckets[p],
-                                         (Xyzz*)partials, queue, acc_blocks, quad_blocks, st));
-        MZK_TRY(ctx->phase_end(st));
-        MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
-        MZK_CUDA_CHECK(launch_fixup(off, sh.keys, (Xyzz*)buckets[p], (const Xyzz*)partials, queue, acc_blocks,
-                                    quad_blocks, (uint32_t)ctx->num_sms * 2, st));
-        ctx->launches += 3;
-        MZK_TRY(ctx->phase_end(st));
+        const Accumulation acc{ba + part.begin, (const uint32_t*)sorted, off, sh.keys, (Xyzz*)buckets[p],
+                               (Xyzz*)partials, queue, acc_blocks, quad_blocks, (uint32_t)ctx->num_sms * 2};
+        std::vector<KeyRange> ranges;
+        for (int w = 0; w < sh.windows; w++) ranges.push_back({(uint32_t)(w + 1) * sh.nb, np});
+        MZK_TRY(accumulate(ctx, acc, ranges, (uint64_t)sh.windows * np, host_entries + p, st));
         MZK_CUDA_CHECK(cudaMemcpyAsync(host_entries + p, off + sh.keys, 4, cudaMemcpyDeviceToHost, st));
     }
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
@@ -1272,7 +1601,7 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
         return ERR_ARG;
     }
     int acc_blocks_per_sm = 0;
-    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&acc_blocks_per_sm, k_accumulate, kAccThreads, 0));
+    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&acc_blocks_per_sm, k_accumulate<true>, kAccThreads, 0));
     if (acc_blocks_per_sm < 1) acc_blocks_per_sm = 1;
     const uint32_t acc_blocks = (uint32_t)(ctx->num_sms * acc_blocks_per_sm);
     const uint32_t acc_threads = acc_blocks * kAccThreads;
@@ -1329,16 +1658,14 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
         MZK_LAUNCH_CHECK(ctx);
     }
     MZK_TRY(ctx->phase_end(st));
-    MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
-    MZK_CUDA_CHECK(launch_accumulate(static_cast<const Affine*>(d_bases), (const uint32_t*)sorted,
-                                     (const uint32_t*)offsets, (uint32_t)keys, (Xyzz*)buckets, (Xyzz*)partials, queue,
-                                     acc_blocks, quad_blocks, st));
-    MZK_TRY(ctx->phase_end(st));
-    MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
-    MZK_CUDA_CHECK(launch_fixup((const uint32_t*)offsets, (uint32_t)keys, (Xyzz*)buckets, (const Xyzz*)partials,
-                                queue, acc_blocks, quad_blocks, (uint32_t)ctx->num_sms * 2, st));
-    ctx->launches += 3;
-    MZK_TRY(ctx->phase_end(st));
+    const Accumulation acc{static_cast<const Affine*>(d_bases), (const uint32_t*)sorted, (const uint32_t*)offsets,
+                           (uint32_t)keys, (Xyzz*)buckets, (Xyzz*)partials, queue, acc_blocks, quad_blocks,
+                           (uint32_t)ctx->num_sms * 2};
+    std::vector<KeyRange> ranges;
+    for (const BatchItemDev& it : hi)
+        for (uint32_t w = 0; w < (it.fixed ? 1u : it.windows); w++)
+            ranges.push_back({it.key_start + (w + 1) * it.nb, (uint64_t)it.n * (it.fixed ? it.windows : 1u)});
+    MZK_TRY(accumulate(ctx, acc, ranges, entries, static_cast<uint32_t*>(host_wsum), st));
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
     const BucketSets sets{{(const Xyzz*)buckets}, {(const uint32_t*)offsets}, 1};
     MZK_CUDA_CHECK(launch_reduce(plan, sets, d_tab, (Xyzz*)arena, (Xyzz*)wsum, &ctx->launches, st));
@@ -1439,7 +1766,7 @@ int g_noalloc_sms[kNoAllocMaxDevices] = {};
 // exclusive scan into caller-provided tile sums (no allocation)
 Status scan_u32_noalloc(const uint32_t* in, uint32_t* out, uint32_t len, uint32_t* sums, cudaStream_t st) {
     const uint32_t tiles = (len + kScanTile - 1) / kScanTile;
-    k_scan_tiles<<<tiles, kScanThreads, 0, st>>>(in, out, len, sums);
+    k_scan_tiles<false><<<tiles, kScanThreads, 0, st>>>(in, out, len, sums);
     MZK_CUDA_CHECK(cudaGetLastError());
     k_scan_sums<<<1, kScanThreads, 0, st>>>(sums, tiles);
     MZK_CUDA_CHECK(cudaGetLastError());
@@ -1517,8 +1844,10 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
     k_scatter<<<pt_blocks, pt_threads, 0, st>>>(sc, n, sh.c, sh.windows, sh.nb, offsets + 1, sorted);
     MZK_CUDA_CHECK(cudaGetLastError());
     // (by lanes: the fixed grid of 64 blocks holds 2048 quads only)
-    MZK_CUDA_CHECK(launch_accumulate(ba, sorted, offsets, sh.keys, buckets, partials, queue, kNoAllocAccBlocks, 0, st));
-    MZK_CUDA_CHECK(launch_fixup(offsets, sh.keys, buckets, partials, queue, kNoAllocAccBlocks, 0, kNoAllocAccBlocks, st));
+    const Accumulation job{ba,       sorted, offsets, sh.keys, buckets, partials, queue, kNoAllocAccBlocks, 0,
+                           kNoAllocAccBlocks};
+    MZK_CUDA_CHECK(launch_accumulate(job, true, st));
+    MZK_CUDA_CHECK(launch_fixup(job, st));
     // the reduction's tables (a copy from pageable memory is staged before the call returns)
     std::vector<Window> wins;
     append_windows(sh, 0, sh.windows, wins);

@@ -87,3 +87,28 @@ def test_accumulation_by_quads_and_by_lanes(ctx, n, sparse):
     finally:
         ctx.set_msm_window(0)
     assert np.array_equal(mzk.affine(got), O.msm_best(s, b))
+
+
+# 2^20 points of width 13: 20 M digits over 81920 buckets, three rounds of pair sums before the mixed additions
+@pytest.mark.parametrize("kind", ["uniform", "pairs"])
+def test_pair_sums(ctx, kind):
+    n = 1 << 20
+    ds, db = ctx.gen_rand_fr(23, n), ctx.gen_bases(29, n)
+    if kind == "pairs":  # neighbours in a bucket: equal (doublings), opposite (infinity), and identity points
+        s, b = ds.download((n, 4)), db.download((n, 12))
+        s[1::4], s[3::4] = s[0::4], s[2::4]
+        b[1::4] = b[0::4]
+        b[3::4, :6], b[3::4, 6:] = b[2::4, :6], b[2::4, 6:]
+        b[7::64] = np.stack([negated(p) for p in b[6::64]])
+        b[8::64] = 0
+        ds.upload(s)
+        db.upload(b)
+    ctx.set_msm_window(13)
+    try:
+        paired = ctx.msm_device(ds, db, n)
+    finally:
+        ctx.set_msm_window(0)
+    # the same MSM in slices too short for pair sums
+    m = 1 << 16
+    parts = [ctx.msm_device(ds.ptr + i * 32, db.ptr + i * 96, m) for i in range(0, n, m)]
+    assert np.array_equal(paired, mzk.g1_sum(np.stack(parts)))
