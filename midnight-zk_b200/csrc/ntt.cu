@@ -6,8 +6,8 @@
 // under them (curves/src/fft.rs:56-198).  Outputs are the same field elements
 // (an NTT has exactly one result), computed by a different schedule:
 //
-//  * passes of radix 2^r (r <= 11) decimation-in-frequency: a block loads a
-//    tile of 2048 elements = 2^r rows x (2048 / 2^r) columns, runs r radix-2
+//  * passes of radix 2^r decimation-in-frequency: a block loads a tile of 2048
+//    elements (256 where a launch is small) = 2^r rows x (2048 / 2^r) columns, runs r radix-2
 //    Gentleman-Sande stages in shared memory, multiplies row k1 of column j by
 //    the inter-pass twiddle w_S^(j*k1) and stores in place.  log2 n = 24 takes
 //    three passes (8 + 8 + 8), 2^26 three (9 + 9 + 8).  Natural order in,
@@ -36,10 +36,11 @@ namespace mzk {
 
 namespace {
 
-constexpr uint32_t kTileLog = 11;
-constexpr uint32_t kTile = 1u << kTileLog;  // elements per block
-constexpr int kNttThreads = 256;
-static_assert(kTile % kNttThreads == 0, "a tile is a whole number of elements per thread");
+// Elements per block: 2^11 by 256 threads, eight elements each in registers
+// for three stages at a time; or 2^8 by 128 threads, one butterfly each, for
+// launches too small to fill the GPU with the former (tile_log_for).
+constexpr uint32_t kTileLog = 11, kSmallTileLog = 8;
+constexpr int kNttThreads = 256, kNttSmallThreads = 128;
 constexpr uint32_t kLoBits = 12;            // low table: w^i for i < 4096
 
 // w^e from the split tables (e < N)
@@ -149,7 +150,10 @@ __device__ __forceinline__ void dif_round(const FrPlanes& sx, const FrPlanes& sw
     }
 }
 
-__global__ void __launch_bounds__(kNttThreads, 2) k_ntt_dif_pass(PassArgs a) {
+template <uint32_t kLog, int kThreads, uint32_t kStages>
+__global__ void __launch_bounds__(kThreads, 2) k_ntt_dif_pass(PassArgs a) {
+    constexpr uint32_t kTile = 1u << kLog;
+    static_assert(kTile % kThreads == 0, "a tile is a whole number of elements per thread");
     extern __shared__ uint4 smem_raw[];
     const uint32_t N = 1u << a.log_n;
     const uint32_t R = 1u << a.log_r;
@@ -169,12 +173,12 @@ __global__ void __launch_bounds__(kNttThreads, 2) k_ntt_dif_pass(PassArgs a) {
     for (uint32_t u = threadIdx.x; u < R / 2; u += blockDim.x)
         sw.set(tw_swz(u), root_pow(a.tlo, a.thi, u << (a.log_n - a.log_r)));
     // all of a thread's global loads are issued before the first is used
-    constexpr int kPer = kTile / kNttThreads;
+    constexpr int kPer = kTile / kThreads;
     Fr v[kPer];
     uint32_t vidx[kPer];
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
-        const uint32_t e = threadIdx.x + (uint32_t)q * kNttThreads;
+        const uint32_t e = threadIdx.x + (uint32_t)q * kThreads;
         const uint32_t m = e >> log_b, b = e & (B - 1);
         const uint32_t c = c0 + (b << cstep_log);
         vidx[q] = ((c >> log_m) << a.log_s) + (m << log_m) + (c & ((1u << log_m) - 1));
@@ -183,7 +187,7 @@ __global__ void __launch_bounds__(kNttThreads, 2) k_ntt_dif_pass(PassArgs a) {
     }
 #pragma unroll
     for (int q = 0; q < kPer; q++) {
-        const uint32_t e = threadIdx.x + (uint32_t)q * kNttThreads;
+        const uint32_t e = threadIdx.x + (uint32_t)q * kThreads;
         if (e >= tile) continue;
         if (a.use_pre && vidx[q] < a.n_real) {
             const uint32_t r3 = vidx[q] % 3;
@@ -192,14 +196,14 @@ __global__ void __launch_bounds__(kNttThreads, 2) k_ntt_dif_pass(PassArgs a) {
         sx.set(swz(e), v[q]);
     }
     __syncthreads();
-    // stages in rounds of three (radix 8), the last round of one or two
+    // stages in rounds of kStages (three: radix 8), the last round of what is left
     for (uint32_t s = 0; s < a.log_r;) {
-        const uint32_t k = min(3u, a.log_r - s);
+        const uint32_t k = min(kStages, a.log_r - s);
         const bool last = s + k == a.log_r;
-        if (k == 3) {
+        if (kStages >= 3 && k == 3) {
             if (last) dif_round<3, true>(sx, sw, s, a.log_r, log_b, tile);
             else dif_round<3, false>(sx, sw, s, a.log_r, log_b, tile);
-        } else if (k == 2) {
+        } else if (kStages >= 2 && k == 2) {
             if (last) dif_round<2, true>(sx, sw, s, a.log_r, log_b, tile);
             else dif_round<2, false>(sx, sw, s, a.log_r, log_b, tile);
         } else {
@@ -298,8 +302,8 @@ uint32_t grid_for(Context* ctx, uint32_t n, uint32_t threads) {
 // log2 of the rows of each pass of a transform of 2^log_n elements under a
 // split mode: every pass keeps at least one stage and at most the tile's;
 // the remaining passes can always take what is left
-static std::vector<uint32_t> pass_logs(uint32_t log_n, int split) {
-    const uint32_t tile_log = std::min(kTileLog, log_n);
+static std::vector<uint32_t> pass_logs(uint32_t log_n, int split, uint32_t max_tile_log) {
+    const uint32_t tile_log = std::min(max_tile_log, log_n);
     const uint32_t passes = (log_n + tile_log - 1) / tile_log;
     std::vector<uint32_t> logs;
     uint32_t log_s = log_n;
@@ -313,6 +317,18 @@ static std::vector<uint32_t> pass_logs(uint32_t log_n, int split) {
     }
     return logs;
 }
+
+// log2 of the elements per block for `elements` elements in one launch.  A
+// launch of few blocks is bound by the chain of products of one thread: three
+// stages over eight elements are 12 products of ~0.4 us, where 128 threads
+// with a butterfly each need one per stage, and 2^12 elements are 16 blocks
+// instead of 2.  Per call, large tile / small tile: one transform of 2^8 43 / 30
+// us, 2^12 88 / 38, 2^16 101 / 54, 2^17 104 / 70, 2^18 104 / 94; seven of 2^14 105
+// / 67.  At 7 x 2^16 both take 152 us, and beyond the smaller passes only add
+// memory traffic (three passes where the large tile needs two).
+constexpr uint64_t kSmallElements = 1u << 18;
+
+static uint32_t tile_log_for(uint64_t elements) { return elements <= kSmallElements ? kSmallTileLog : kTileLog; }
 
 static int split_of(const Context* ctx, uint32_t log_n) {
     return log_n < (uint32_t)kTuneSlots ? ctx->tuned_ntt_split[log_n] : 0;
@@ -342,6 +358,7 @@ static const Fr* pass_twiddles(Context* ctx, const Domain* d, int root, uint32_t
         return nullptr;
     }
     ctx->launches++;
+    d->pass_tw_mem.push_back(p);
     d->pass_tw[key] = p;
     return p;
 }
@@ -349,7 +366,7 @@ static const Fr* pass_twiddles(Context* ctx, const Domain* d, int root, uint32_t
 Domain::~Domain() {
     for (auto& t : tables)
         if (t) cudaFree(t);
-    for (auto& kv : pass_tw) cudaFree(kv.second);
+    for (void* p : pass_tw_mem) cudaFree(p);
     if (d_tinv) cudaFree(d_tinv);
 }
 
@@ -357,8 +374,9 @@ Domain::~Domain() {
 Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
     // the pass kernel's shared memory limit, set here once rather than per
     // transform: transforms may be captured into CUDA graphs
-    MZK_CUDA_CHECK(cudaFuncSetAttribute(k_ntt_dif_pass, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(kTile * sizeof(Fr) + kTile / 2 * sizeof(Fr))));
+    MZK_CUDA_CHECK(cudaFuncSetAttribute(k_ntt_dif_pass<kTileLog, kNttThreads, 3>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)((1u << kTileLog) * sizeof(Fr) + (1u << kTileLog) / 2 * sizeof(Fr))));
     *out = nullptr;
     if (j < 2 || k < 1 || k > 28) {
         set_error("domain: need j >= 2 and 1 <= k <= 28");
@@ -421,25 +439,54 @@ Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
         k_pow_table<<<grid_for(ctx, hi, 128), 128, 0, ctx->stream>>>(to_dev(w4096), hi, d->hi[r]);
         MZK_LAUNCH_CHECK(ctx);
     }
+    // the pass twiddle tables of the splits in force for each root's size, in
+    // one allocation (without memory for it transforms form their twiddles)
+    struct Table {
+        int root;
+        uint32_t log_n, log_s, log_r;
+    };
+    std::vector<Table> tw;
+    size_t tw_elements = 0;
+    for (int r = 0; r < 4; r++) {
+        const uint32_t log_n = logs[r];
+        for (const uint32_t tile_log : {kTileLog, kSmallTileLog}) {
+            if (tile_log == kSmallTileLog && tile_log_for(1ull << log_n) != kSmallTileLog) continue;
+            const std::vector<uint32_t> pl = pass_logs(log_n, split_of(ctx, log_n), tile_log);
+            uint32_t log_s = log_n;
+            for (size_t p = 0; p + 1 < pl.size(); p++) {
+                bool known = false;
+                for (const Table& t : tw) known = known || (t.root == r && t.log_s == log_s && t.log_r == pl[p]);
+                if (!known) {
+                    tw.push_back({r, log_n, log_s, pl[p]});
+                    tw_elements += (size_t)1 << log_s;
+                }
+                log_s -= pl[p];
+            }
+        }
+    }
+    Fr* tw_mem = nullptr;
+    if (tw_elements && cudaMalloc(&tw_mem, tw_elements * sizeof(Fr)) == cudaSuccess) {
+        d->pass_tw_mem.push_back(tw_mem);
+        for (const Table& t : tw) {
+            k_pass_twiddles<<<grid_for(ctx, 1u << t.log_s, 256), 256, 0, ctx->stream>>>(
+                d->lo[t.root], d->hi[t.root], t.log_n, t.log_s, t.log_r, tw_mem);
+            MZK_LAUNCH_CHECK(ctx);
+            d->pass_tw[std::make_tuple(t.root, t.log_s, t.log_r)] = tw_mem;
+            tw_mem += (size_t)1 << t.log_s;
+        }
+    } else {
+        cudaGetLastError();
+    }
     {
         cudaError_t e = cudaMalloc(&d->d_tinv, (size_t)tlen * sizeof(Fr));
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d->d_tinv, d->t_inv.data(), (size_t)tlen * 32, cudaMemcpyHostToDevice, ctx->stream);
+        // every table is ready for any stream from here on
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) {
             delete d;
             set_error(std::string("domain set-up: ") + cudaGetErrorString(e));
             return ERR_CUDA;
-        }
-    }
-    // the pass twiddle tables of the split in force for each root's size
-    for (int r = 0; r < 4; r++) {
-        const uint32_t log_n = logs[r];
-        const std::vector<uint32_t> pl = pass_logs(log_n, split_of(ctx, log_n));
-        uint32_t log_s = log_n;
-        for (size_t p = 0; p + 1 < pl.size(); p++) {
-            pass_twiddles(ctx, d, r, log_n, log_s, pl[p], ctx->stream);
-            log_s -= pl[p];
         }
     }
     *out = d;
@@ -454,17 +501,18 @@ Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
 // (times post[i % 3] when post is given, only positions < m_out).  Since
 // that pass's writes cross blocks, it reads from the scratch the earlier
 // passes wrote, so in[t] and out[t] may be the same buffer.  A transform of
-// one tile (log_n <= 11) is one block, which reads all before it writes.
+// one tile is one block, which reads all before it writes.
 static Status dif_passes(Context* ctx, const Domain* d, int root, uint32_t log_n, const Fr* const* in,
                          Fr* const* out, uint32_t T, uint32_t n_real, bool coset, const host::Fr4* post,
                          uint32_t m_out, cudaStream_t st) {
     const uint32_t N = 1u << log_n;
-    const uint32_t tile = std::min(kTile, N);
-    const std::vector<uint32_t> logs = pass_logs(log_n, split_of(ctx, log_n));
-    const uint32_t passes = (uint32_t)logs.size();
     // transforms per launch: at most kNttBatch and 2^25 elements of scratch
     // (large transforms fill the GPU alone)
     const uint32_t TB = std::min({T, kNttBatch, std::max(1u, (1u << 25) >> log_n)});
+    const uint32_t tile_log = tile_log_for((uint64_t)TB << log_n);
+    const uint32_t tile = std::min(1u << tile_log, N);
+    const std::vector<uint32_t> logs = pass_logs(log_n, split_of(ctx, log_n), tile_log);
+    const uint32_t passes = (uint32_t)logs.size();
     Fr* tmp = nullptr;
     if (passes > 1) {
         void* p;
@@ -499,7 +547,9 @@ static Status dif_passes(Context* ctx, const Domain* d, int root, uint32_t log_n
             a.m_out = m_out;
             for (int i = 0; i < 3; i++) a.post[i] = to_dev(post ? post[i] : host::fr_one());
             const size_t smem = (size_t)tile * sizeof(Fr) + (size_t)(1u << log_r) / 2 * sizeof(Fr);
-            k_ntt_dif_pass<<<dim3(N / tile, tb), kNttThreads, smem, st>>>(a);
+            const dim3 grid(N / tile, tb);
+            if (tile_log == kTileLog) k_ntt_dif_pass<kTileLog, kNttThreads, 3><<<grid, kNttThreads, smem, st>>>(a);
+            else k_ntt_dif_pass<kSmallTileLog, kNttSmallThreads, 1><<<grid, kNttSmallThreads, smem, st>>>(a);
             MZK_LAUNCH_CHECK(ctx);
             log_s -= log_r;
         }

@@ -42,10 +42,12 @@ struct Domain {
     // writes its output: tw[(m << (log_s - log_r)) + j] = w^((N/S) j bitrev_r(m))
     // for the pass over segments of S = 2^log_s elements with R = 2^log_r rows
     // (N = 2^log_n of root r).  Keyed by (root, log_s, log_r); built for the
-    // split in force when the domain is created, and for another split the
-    // first time a transform outside stream capture uses it.
+    // splits in force (both tile sizes) when the domain is created, in one
+    // allocation, and for another split the first time a transform outside
+    // stream capture uses it.
     mutable std::mutex tw_mu;
     mutable std::map<std::tuple<int, uint32_t, uint32_t>, Fr*> pass_tw;
+    mutable std::vector<void*> pass_tw_mem;  // the tables' allocations
     ~Domain();
 };
 
