@@ -33,10 +33,9 @@ namespace mzk {
 namespace {
 
 constexpr int kThreads = 256;
-// elements per thread of a linear recurrence: up to 64, fewer when n is too
-// small to give every SM work (each thread's chunk is a serial chain)
-constexpr uint32_t kRecChunkMax = 64, kRecChunkMin = 4;
-constexpr uint32_t kScanItems = 8;  // elements per thread of a block scan
+// elements per thread of a block scan: two serial chains of as many products,
+// so fewer where the tiles do not fill the GPU
+constexpr uint32_t kScanItemsMin = 2, kScanItemsMax = 8;
 constexpr uint32_t kMaxPermSetCols = 8;
 constexpr uint32_t kMaxLogupChunks = 8;
 
@@ -91,132 +90,93 @@ __device__ Fr block_exclusive(Fr v, Fr* sm, Fr* total) {
     return ex;
 }
 
-// block-wide exclusive suffix product of one value per thread: the product of
-// the values of the threads above this one
-__device__ Fr block_exclusive_suffix_product(Fr v, Fr* sm) {
-    sm[threadIdx.x] = v;
-    __syncthreads();
-    for (uint32_t off = 1; off < blockDim.x; off <<= 1) {
-        Fr o = fr_one();
-        if (threadIdx.x + off < blockDim.x) o = sm[threadIdx.x + off];
-        __syncthreads();
-        if (threadIdx.x + off < blockDim.x) sm[threadIdx.x] = fr_mul(o, sm[threadIdx.x]);
-        __syncthreads();
-    }
-    const Fr ex = threadIdx.x + 1 < blockDim.x ? sm[threadIdx.x + 1] : fr_one();
-    __syncthreads();
-    return ex;
-}
-
-// ---- batch inversion (ff BatchInvert: zeros stay zero): a block takes
-// kThreads x C consecutive elements (thread t the elements t, t + kThreads,
-// ... of the block's range, so loads and stores are coalesced), each thread
-// multiplies its C non-zero elements in registers, the block combines the
-// threads' products by a prefix and a suffix scan in shared memory, and the
-// inverse of the block's total gives every thread the inverse of its product
-// (prefix x suffix x 1/total); the backward pass then inverts each element.
-// The inverse of the total is one inversion by one thread of the block (17.6
-// us; by binary extended Euclid it took 54) when the blocks fit one wave on the
-// GPU; otherwise the totals are batch-inverted first (k_invert_totals, then
-// this function on the totals), since a serial inversion per block would leave
-// the SMs idle wave after wave.
-constexpr int kInvPerThread = 4;
+// ---- batch inversion (ff BatchInvert: zeros stay zero) ----
+//
+// A thread multiplies C elements (one from each of C rows of gridDim x
+// blockDim, so that loads and stores are coalesced), inverts the product and
+// works backward; zeros are left out.  The inversion (inv_divsteps) takes a warp
+// the same time for 1 value as for 32, 17 us alone on its scheduler and ~13 us
+// for each warp where there are several, so every thread has its own and
+// nothing is exchanged: one inversion per block between two scans over its
+// threads took 52 us for 2^16 elements and 94 for 2^18.  C weighs the inversions
+// against the chain of 3 C products (0.3..0.5 us each): up to 8 keeps the
+// elements in registers, 16 reads them twice.
+constexpr int kInvThreads = 128;
 
 template <int C>
-__global__ void __launch_bounds__(kThreads) k_invert_totals(const Fr* __restrict__ a, uint64_t n, Fr* __restrict__ tot) {
-    __shared__ Fr sm[kThreads];
-    const uint64_t base = (uint64_t)blockIdx.x * kThreads * C + threadIdx.x;
-    Fr acc = fr_one();
+__global__ void __launch_bounds__(kInvThreads, C > 8 ? 4 : 3) k_batch_invert(Fr* __restrict__ a, uint64_t n) {
+    constexpr bool kKeep = C <= 8;
+    const uint64_t row = (uint64_t)gridDim.x * kInvThreads, first = (uint64_t)blockIdx.x * kInvThreads + threadIdx.x;
+    Fr pre[C], kept[kKeep ? C : 1];
+    if (kKeep) {
 #pragma unroll
-    for (int k = 0; k < C; k++) {
-        const uint64_t i = base + (uint64_t)k * kThreads;
-        if (i < n) {
-            const Fr v = a[i];
-            if (!fr_is_zero(v)) acc = fr_mul(acc, v);
+        for (int k = 0; k < C; k++) {
+            const uint64_t i = first + (uint64_t)k * row;
+            kept[kKeep ? k : 0] = i < n ? a[i] : fr_zero();
         }
     }
-    Fr total;
-    block_exclusive<true>(acc, sm, &total);
-    if (threadIdx.x == 0) tot[blockIdx.x] = total;  // non-zero: a product of non-zero elements (or one)
-}
-
-template <int C, bool kGivenInverse>
-__global__ void __launch_bounds__(kThreads) k_batch_invert(Fr* __restrict__ a, uint64_t n,
-                                                           const Fr* __restrict__ tot_inv) {
-    __shared__ Fr sm[kThreads];
-    __shared__ Fr total_inv;
-    const uint64_t base = (uint64_t)blockIdx.x * kThreads * C + threadIdx.x;
-    Fr v[C], pre[C];
-#pragma unroll
-    for (int k = 0; k < C; k++) {
-        const uint64_t i = base + (uint64_t)k * kThreads;
-        v[k] = i < n ? a[i] : fr_zero();
-    }
+    auto element = [&](int k) {
+        if (kKeep) return kept[kKeep ? k : 0];
+        const uint64_t i = first + (uint64_t)k * row;
+        return i < n ? a[i] : fr_zero();
+    };
     Fr acc = fr_one();
 #pragma unroll
     for (int k = 0; k < C; k++) {
+        const Fr v = element(k);
         pre[k] = acc;
-        if (!fr_is_zero(v[k])) acc = fr_mul(acc, v[k]);
+        if (!fr_is_zero(v)) acc = fr_mul(acc, v);
     }
-    Fr total;
-    const Fr below = block_exclusive<true>(acc, sm, &total);
-    const Fr above = block_exclusive_suffix_product(acc, sm);
-    if (threadIdx.x == 0) total_inv = kGivenInverse ? tot_inv[blockIdx.x] : fr_invert(total);
-    __syncthreads();
-    Fr inv = fr_mul(fr_mul(total_inv, below), above);  // 1 / acc
+    Fr inv = fr_invert(acc);
 #pragma unroll
     for (int k = C - 1; k >= 0; k--) {
-        const uint64_t i = base + (uint64_t)k * kThreads;
-        if (!fr_is_zero(v[k])) {
-            if (i < n) a[i] = fr_mul(pre[k], inv);
-            inv = fr_mul(inv, v[k]);
+        const Fr v = element(k);
+        if (!fr_is_zero(v)) {
+            a[first + (uint64_t)k * row] = fr_mul(pre[k], inv);
+            inv = fr_mul(inv, v);
         }
     }
 }
 
-Status batch_invert_level(Context* ctx, Fr* a, uint64_t n, cudaStream_t st, int level) {
+Status batch_invert(Context* ctx, Fr* a, uint64_t n, cudaStream_t st) {
     if (n == 0) return OK;
-    const uint64_t per = (uint64_t)kThreads * kInvPerThread;
-    const uint64_t blocks = (n + per - 1) / per;
-    if (blocks <= (uint64_t)ctx->num_sms * 2) {  // one wave at 2 blocks per SM
-        k_batch_invert<kInvPerThread, false><<<(uint32_t)blocks, kThreads, 0, st>>>(a, n, nullptr);
-        MZK_LAUNCH_CHECK(ctx);
-        return OK;
-    }
-    if (level >= 4) {
+    // one warp per scheduler up to C = 8 (2^17 elements), two at 2^18
+    const uint64_t wave = (uint64_t)ctx->num_sms * kInvThreads;
+    const uint64_t per = (n + wave - 1) / wave;
+    const int C = per <= 1 ? 1 : per <= 2 ? 2 : per <= 4 ? 4 : per <= 16 ? 8 : 16;
+    const uint64_t blocks = (n + (uint64_t)kInvThreads * C - 1) / ((uint64_t)kInvThreads * C);
+    if (blocks > 0x7fffffffull) {
         set_error("batch_invert: too many elements");
         return ERR_ARG;
     }
-    static const char* const kTotNames[4] = {"grand_inv_tot0", "grand_inv_tot1", "grand_inv_tot2", "grand_inv_tot3"};
-    void* buf;
-    MZK_TRY(ctx->ensure(kTotNames[level], blocks * sizeof(Fr), &buf));
-    Fr* tot = static_cast<Fr*>(buf);
-    k_invert_totals<kInvPerThread><<<(uint32_t)blocks, kThreads, 0, st>>>(a, n, tot);
-    MZK_LAUNCH_CHECK(ctx);
-    MZK_TRY(batch_invert_level(ctx, tot, blocks, st, level + 1));
-    k_batch_invert<kInvPerThread, true><<<(uint32_t)blocks, kThreads, 0, st>>>(a, n, tot);
+    const uint32_t g = (uint32_t)blocks;
+    switch (C) {
+        case 1: k_batch_invert<1><<<g, kInvThreads, 0, st>>>(a, n); break;
+        case 2: k_batch_invert<2><<<g, kInvThreads, 0, st>>>(a, n); break;
+        case 4: k_batch_invert<4><<<g, kInvThreads, 0, st>>>(a, n); break;
+        case 8: k_batch_invert<8><<<g, kInvThreads, 0, st>>>(a, n); break;
+        default: k_batch_invert<16><<<g, kInvThreads, 0, st>>>(a, n); break;
+    }
     MZK_LAUNCH_CHECK(ctx);
     return OK;
 }
 
-Status batch_invert(Context* ctx, Fr* a, uint64_t n, cudaStream_t st) { return batch_invert_level(ctx, a, n, st, 0); }
-
-// pass 1: out = exclusive scan within each tile of kThreads * kScanItems, sums[tile] = tile total
-template <bool kMul>
+// pass 1: out = exclusive scan within each tile of kThreads * kItems, sums[tile] = tile total
+template <bool kMul, uint32_t kItems>
 __global__ void __launch_bounds__(kThreads) k_scan_tile(const Fr* in, Fr* out, uint64_t n, Fr* __restrict__ sums) {
     __shared__ Fr sm[kThreads];
-    const uint64_t base = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * kScanItems;
-    Fr v[kScanItems];
+    const uint64_t base = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * kItems;
+    Fr v[kItems];
     Fr acc = identity<kMul>();
 #pragma unroll
-    for (uint32_t j = 0; j < kScanItems; j++) {
+    for (uint32_t j = 0; j < kItems; j++) {
         v[j] = base + j < n ? in[base + j] : identity<kMul>();
         acc = op<kMul>(acc, v[j]);
     }
     Fr total;
     Fr pre = block_exclusive<kMul>(acc, sm, &total);
 #pragma unroll
-    for (uint32_t j = 0; j < kScanItems; j++) {
+    for (uint32_t j = 0; j < kItems; j++) {
         if (base + j < n) out[base + j] = pre;
         pre = op<kMul>(pre, v[j]);
     }
@@ -225,8 +185,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_tile(const Fr* in, Fr* out, u
 
 // pass 3: out[i] = prefix[tile] (op) out[i]
 template <bool kMul>
-__global__ void k_scan_apply(Fr* __restrict__ out, uint64_t n, const Fr* __restrict__ prefix) {
-    const uint64_t tile = (uint64_t)kThreads * kScanItems;
+__global__ void k_scan_apply(Fr* __restrict__ out, uint64_t n, const Fr* __restrict__ prefix, uint64_t tile) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint64_t t = i / tile;
@@ -238,158 +197,192 @@ __global__ void k_scan_apply(Fr* __restrict__ out, uint64_t n, const Fr* __restr
 template <bool kMul>
 Status scan_exclusive(Context* ctx, const Fr* in, Fr* out, uint64_t n, cudaStream_t st, int depth = 0) {
     if (n == 0) return OK;
-    const uint64_t tile = (uint64_t)kThreads * kScanItems;
+    uint32_t items = kScanItemsMin;
+    while (items < kScanItemsMax && n / (kThreads * items * 2) >= (uint64_t)ctx->num_sms * 2) items *= 2;
+    const uint64_t tile = (uint64_t)kThreads * items;
     const uint64_t tiles = (n + tile - 1) / tile;
     void* sums;
     MZK_TRY(ctx->ensure(("grand_scan_" + std::to_string(depth)).c_str(), (tiles + 1) * sizeof(Fr), &sums));
-    k_scan_tile<kMul><<<(uint32_t)tiles, kThreads, 0, st>>>(in, out, n, (Fr*)sums);
+    if (items == 2) k_scan_tile<kMul, 2><<<(uint32_t)tiles, kThreads, 0, st>>>(in, out, n, (Fr*)sums);
+    else if (items == 4) k_scan_tile<kMul, 4><<<(uint32_t)tiles, kThreads, 0, st>>>(in, out, n, (Fr*)sums);
+    else k_scan_tile<kMul, 8><<<(uint32_t)tiles, kThreads, 0, st>>>(in, out, n, (Fr*)sums);
     MZK_LAUNCH_CHECK(ctx);
     if (tiles > 1) {
         // exclusive scan of the tile totals (recursively), then fold it in
         MZK_TRY(scan_exclusive<kMul>(ctx, (const Fr*)sums, (Fr*)sums, tiles, st, depth + 1));
-        k_scan_apply<kMul><<<grid_for(ctx, n, kThreads), kThreads, 0, st>>>(out, n, (const Fr*)sums);
+        k_scan_apply<kMul><<<grid_for(ctx, n, kThreads), kThreads, 0, st>>>(out, n, (const Fr*)sums, tile);
         MZK_LAUNCH_CHECK(ctx);
     }
     return OK;
 }
 
-// ---- first-order linear recurrence from the top: y_i = c_i + k y_{i+1},
-// y_n = 0.  Thread t solves its chunk [tK, tK+K) with a zero carry-in and
-// records L_t = its local y at tK; the true values at the chunk starts solve
-// the same recurrence over the L_t with k^K; a last pass adds k^(hi-i) Y_{t+1}.
-__global__ void __launch_bounds__(kThreads) k_rec_local(const Fr* __restrict__ c, Fr* __restrict__ y, uint64_t n,
-                                                        Fr k, Fr* __restrict__ lows, uint32_t K) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t lo = t * K;
-    if (lo >= n) return;
-    const uint64_t hi = min(n, lo + K);
-    Fr acc = fr_zero();
-    for (uint64_t i = hi; i-- > lo;) {
-        acc = fr_add(c[i], fr_mul(k, acc));
-        y[i] = acc;
-    }
-    lows[t] = acc;
-}
-__global__ void __launch_bounds__(kThreads) k_rec_fix(Fr* __restrict__ y, uint64_t n, Fr k,
-                                                      const Fr* __restrict__ starts, uint64_t chunks, uint32_t K) {
-    const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t + 1 >= chunks) return;  // the top chunk has a zero carry-in
-    const uint64_t lo = t * K, hi = lo + K;
-    const Fr carry = starts[t + 1];
-    Fr pw = k;  // k^(hi - i) for i = hi - 1
-    for (uint64_t i = hi; i-- > lo;) {
-        y[i] = fr_add(y[i], fr_mul(pw, carry));
-        pw = fr_mul(pw, k);
-    }
-}
-
-// y (n) from c (n), in and out may not alias
-Status linrec_suffix(Context* ctx, const Fr* c, Fr* y, uint64_t n, const host::Fr4& k, cudaStream_t st, int depth = 0) {
-    if (n == 0) return OK;
-    // the chunk length: 64 while that leaves at least 2 threads of 256 per SM
-    // per warp slot, down to 4 for smaller n; small recursion levels keep 64
-    uint32_t K = kRecChunkMax;
-    const uint64_t want_threads = (uint64_t)ctx->num_sms * kThreads * 2;
-    while (K > kRecChunkMin && n / K < want_threads && n > (uint64_t)kRecChunkMax * kRecChunkMax) K >>= 1;
-    const uint64_t chunks = (n + K - 1) / K;
-    void* lows;
-    MZK_TRY(ctx->ensure(("grand_rec_" + std::to_string(depth)).c_str(), 2 * chunks * sizeof(Fr), &lows));
-    Fr* L = (Fr*)lows;
-    Fr* Y = L + chunks;
-    k_rec_local<<<(uint32_t)((chunks + kThreads - 1) / kThreads), kThreads, 0, st>>>(c, y, n, to_dev(k), L, K);
-    MZK_LAUNCH_CHECK(ctx);
-    if (chunks > 1) {
-        host::Fr4 kk = k;  // k^K
-        for (uint32_t b = 1; b < K; b <<= 1) kk = host::fr_mul(kk, kk);
-        MZK_TRY(linrec_suffix(ctx, L, Y, chunks, kk, st, depth + 1));
-        k_rec_fix<<<(uint32_t)((chunks + kThreads - 1) / kThreads), kThreads, 0, st>>>(y, n, to_dev(k), Y, chunks, K);
-        MZK_LAUNCH_CHECK(ctx);
-    }
-    return OK;
-}
-
-// The same recurrences for T tasks of one length n, blockIdx.y picking the
-// task: its input, output and factor, and its slice of the chunk values.
+// ---- first-order linear recurrences from the top: y_i = c_i + k y_{i+1},
+// y_n = 0, for T tasks of one length (blockIdx.y: the task) ----
+//
+// A block takes kThreads x K consecutive elements, a thread K of them.  The
+// chain of K products gives a thread its y with a zero carry-in, a scan over
+// the block (log2 kThreads products, the factors k^(K 2^l) alike for every
+// thread) the carry from the threads above, and the same chain started from
+// the true carry the outputs.  Between blocks the values at the block starts
+// solve the same recurrence with the factor k^(kThreads K): k_rec_totals leaves
+// them, this function solves them, and k_rec_solve starts from the results.
+// The products of a thread are a serial chain and small inputs are bound by it:
+// K is 4 unless the blocks already fill the GPU.
+constexpr uint32_t kRecItemsMin = 4, kRecItemsMax = 16;
 constexpr uint32_t kRecBatch = 32;
+constexpr uint32_t kRecLevels = 8;  // log2 kThreads
+static_assert((1 << kRecLevels) == kThreads, "one scan level per bit of the thread index");
+
 struct RecTasks {
     const Fr* c[kRecBatch];
     Fr* y[kRecBatch];
     Fr k[kRecBatch];
+    Fr kk[kRecBatch][kRecLevels];  // k^(K 2^l)
 };
-__global__ void __launch_bounds__(kThreads) k_rec_local_batch(const RecTasks t, uint64_t n, Fr* __restrict__ lows,
-                                                              uint64_t chunks, uint32_t K) {
-    const uint32_t j = blockIdx.y;
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t lo = c * K;
-    if (lo >= n) return;
-    const uint64_t hi = min(n, lo + K);
-    const Fr k = t.k[j];
-    const Fr* __restrict__ in = t.c[j];
-    Fr* __restrict__ y = t.y[j];
+
+// the thread's y at its first element with a zero carry-in
+template <uint32_t K>
+__device__ __forceinline__ Fr rec_chain(const Fr* __restrict__ c, uint64_t lo, uint64_t n, const Fr& k) {
     Fr acc = fr_zero();
-    for (uint64_t i = hi; i-- > lo;) {
-        acc = fr_add(in[i], fr_mul(k, acc));
-        y[i] = acc;
+#pragma unroll
+    for (int i = (int)K - 1; i >= 0; i--) {
+        const Fr v = lo + (uint64_t)i < n ? c[lo + (uint64_t)i] : fr_zero();
+        acc = fr_add(v, fr_mul(k, acc));
     }
-    lows[2 * chunks * j + c] = acc;
+    return acc;
 }
-__global__ void __launch_bounds__(kThreads) k_rec_fix_batch(const RecTasks t, uint64_t n, const Fr* __restrict__ lows,
-                                                            uint64_t chunks, uint32_t K) {
+
+// v <- sum_{u >= t} k^(K (u - t)) v_u over the block's threads (sm: kThreads)
+__device__ __forceinline__ Fr rec_scan(Fr v, const Fr* __restrict__ kk, Fr* sm) {
+    sm[threadIdx.x] = v;
+    __syncthreads();
+#pragma unroll 1
+    for (uint32_t l = 0; l < kRecLevels; l++) {
+        const uint32_t off = 1u << l;
+        const bool on = threadIdx.x + off < (uint32_t)kThreads;
+        if (on) v = fr_add(v, fr_mul(kk[l], sm[threadIdx.x + off]));
+        __syncthreads();
+        sm[threadIdx.x] = v;
+        __syncthreads();
+    }
+    return v;
+}
+
+// starts[task * stride + block] = the block's y at its first element with a zero carry-in
+template <uint32_t K>
+__global__ void __launch_bounds__(kThreads) k_rec_totals(const RecTasks t, uint64_t n, Fr* __restrict__ starts,
+                                                         uint64_t stride) {
+    __shared__ Fr sm[kThreads];
     const uint32_t j = blockIdx.y;
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c + 1 >= chunks) return;  // the top chunk has a zero carry-in
-    const uint64_t lo = c * K, hi = lo + K;
-    const Fr k = t.k[j];
-    const Fr carry = lows[2 * chunks * j + chunks + c + 1];  // Y of the chunk above
+    const uint64_t lo = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * K;
+    const Fr v = rec_scan(rec_chain<K>(t.c[j], lo, n, t.k[j]), t.kk[j], sm);
+    if (threadIdx.x == 0) starts[j * stride + blockIdx.x] = v;
+}
+
+// every y, the block's carry-in carry[task * stride + block + 1] (none for the last)
+template <uint32_t K>
+__global__ void __launch_bounds__(kThreads) k_rec_solve(const RecTasks t, uint64_t n, const Fr* __restrict__ carry,
+                                                        uint64_t stride) {
+    __shared__ Fr sm[kThreads];
+    const uint32_t j = blockIdx.y;
+    const Fr* __restrict__ c = t.c[j];
     Fr* __restrict__ y = t.y[j];
-    Fr pw = k;
-    for (uint64_t i = hi; i-- > lo;) {
-        y[i] = fr_add(y[i], fr_mul(pw, carry));
-        pw = fr_mul(pw, k);
+    const Fr k = t.k[j];
+    const uint64_t lo = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * K;
+    Fr v = rec_chain<K>(c, lo, n, k);
+    const bool has_carry = blockIdx.x + 1 < gridDim.x;
+    Fr in = fr_zero();
+    if (has_carry) in = carry[j * stride + blockIdx.x + 1];
+    // the carry enters as the value above the last thread's chunk
+    if (has_carry && threadIdx.x == kThreads - 1) v = fr_add(v, fr_mul(t.kk[j][0], in));
+    rec_scan(v, t.kk[j], sm);
+    Fr acc = threadIdx.x + 1 < (uint32_t)kThreads ? sm[threadIdx.x + 1] : in;
+#pragma unroll
+    for (int i = (int)K - 1; i >= 0; i--) {
+        if (lo + (uint64_t)i < n) {
+            acc = fr_add(c[lo + (uint64_t)i], fr_mul(k, acc));
+            y[lo + (uint64_t)i] = acc;
+        }
     }
 }
 
-// linrec_suffix for T tasks of one length: y[j] (n) from c[j] (n) with
-// factor k[j]; the chunk values of every level sit in one buffer per level
-// (task j: its lows L_j then its starts Y_j)
+template <uint32_t K>
+cudaError_t launch_rec(const RecTasks& t, uint64_t n, uint64_t blocks, uint32_t T, Fr* starts, const Fr* carry,
+                       uint64_t stride, cudaStream_t st) {
+    const dim3 grid((uint32_t)blocks, T);
+    if (starts) k_rec_totals<K><<<grid, kThreads, 0, st>>>(t, n, starts, stride);
+    else k_rec_solve<K><<<grid, kThreads, 0, st>>>(t, n, carry, stride);
+    return cudaGetLastError();
+}
+
+// y[j] (n) from c[j] (n) with factor k[j]; in and out may not alias.
+// first_only: y[j] receives its first value alone (y[j][0]).
 Status linrec_suffix_batch(Context* ctx, const Fr* const* c, Fr* const* y, const host::Fr4* k, uint32_t T, uint64_t n,
-                           cudaStream_t st, int depth = 0) {
+                           cudaStream_t st, bool first_only = false, int depth = 0) {
     if (n == 0 || T == 0) return OK;
-    uint32_t K = kRecChunkMax;
-    const uint64_t want_threads = (uint64_t)ctx->num_sms * kThreads * 2;
-    while (K > kRecChunkMin && n * T / K < want_threads && n > (uint64_t)kRecChunkMax * kRecChunkMax) K >>= 1;
-    const uint64_t chunks = (n + K - 1) / K;
+    // four elements per thread until the tasks' blocks are four per SM
+    uint32_t K = kRecItemsMin;
+    while (K < kRecItemsMax && n * std::min(T, kRecBatch) / ((uint64_t)kThreads * K * 2) >= (uint64_t)ctx->num_sms * 4)
+        K *= 2;
+    const uint64_t blocks = (n + (uint64_t)kThreads * K - 1) / ((uint64_t)kThreads * K);
+    auto launch = [&](const RecTasks& t, uint32_t tb, Fr* starts, const Fr* carry) {
+        return K == 4   ? launch_rec<4>(t, n, blocks, tb, starts, carry, 2 * blocks, st)
+               : K == 8 ? launch_rec<8>(t, n, blocks, tb, starts, carry, 2 * blocks, st)
+                        : launch_rec<16>(t, n, blocks, tb, starts, carry, 2 * blocks, st);
+    };
     for (uint32_t j0 = 0; j0 < T; j0 += kRecBatch) {
         const uint32_t tb = std::min(kRecBatch, T - j0);
-        void* lows;
-        MZK_TRY(ctx->ensure(("grand_recb_" + std::to_string(depth)).c_str(), 2 * chunks * tb * sizeof(Fr), &lows));
-        Fr* L = (Fr*)lows;
         RecTasks t;
+        std::vector<host::Fr4> kblock(tb);
         for (uint32_t j = 0; j < tb; j++) {
             t.c[j] = c[j0 + j];
             t.y[j] = y[j0 + j];
             t.k[j] = to_dev(k[j0 + j]);
-        }
-        const dim3 grid((uint32_t)((chunks + kThreads - 1) / kThreads), tb);
-        k_rec_local_batch<<<grid, kThreads, 0, st>>>(t, n, L, chunks, K);
-        MZK_LAUNCH_CHECK(ctx);
-        if (chunks > 1) {
-            // the chunk starts: the same recurrence over the lows with k^K
-            std::vector<const Fr*> lc(tb);
-            std::vector<Fr*> ly(tb);
-            std::vector<host::Fr4> kk(tb);
-            for (uint32_t j = 0; j < tb; j++) {
-                lc[j] = L + 2 * chunks * j;
-                ly[j] = L + 2 * chunks * j + chunks;
-                kk[j] = k[j0 + j];
-                for (uint32_t b = 1; b < K; b <<= 1) kk[j] = host::fr_mul(kk[j], kk[j]);
+            host::Fr4 p = k[j0 + j];
+            for (uint32_t b = 1; b < K; b <<= 1) p = host::fr_mul(p, p);
+            for (uint32_t l = 0; l < kRecLevels; l++) {
+                t.kk[j][l] = to_dev(p);
+                p = host::fr_mul(p, p);
             }
-            MZK_TRY(linrec_suffix_batch(ctx, lc.data(), ly.data(), kk.data(), tb, chunks, st, depth + 1));
-            k_rec_fix_batch<<<grid, kThreads, 0, st>>>(t, n, L, chunks, K);
-            MZK_LAUNCH_CHECK(ctx);
+            kblock[j] = p;  // k^(kThreads K)
         }
+        Fr* starts = nullptr;
+        if (blocks > 1) {
+            // task j's block values at 2 blocks j, the solved ones after them
+            void* buf;
+            MZK_TRY(ctx->ensure(("grand_rec_" + std::to_string(depth)).c_str(), 2 * blocks * tb * sizeof(Fr), &buf));
+            starts = static_cast<Fr*>(buf);
+            MZK_CUDA_CHECK(launch(t, tb, starts, nullptr));
+            ctx->launches++;
+            std::vector<const Fr*> sc(tb);
+            std::vector<Fr*> sy(tb);
+            for (uint32_t j = 0; j < tb; j++) {
+                sc[j] = starts + 2 * blocks * j;
+                sy[j] = first_only ? t.y[j] : starts + 2 * blocks * j + blocks;
+            }
+            MZK_TRY(linrec_suffix_batch(ctx, sc.data(), sy.data(), kblock.data(), tb, blocks, st, first_only, depth + 1));
+            if (first_only) continue;
+        } else if (first_only) {
+            // one block: its start is the first value
+            for (uint32_t j = 0; j < tb; j++) {
+                RecTasks one = t;
+                one.c[0] = t.c[j];
+                one.k[0] = t.k[j];
+                for (uint32_t l = 0; l < kRecLevels; l++) one.kk[0][l] = t.kk[j][l];
+                MZK_CUDA_CHECK(launch(one, 1, t.y[j], nullptr));
+                ctx->launches++;
+            }
+            continue;
+        }
+        MZK_CUDA_CHECK(launch(t, tb, nullptr, starts ? starts + blocks : nullptr));
+        ctx->launches++;
     }
     return OK;
+}
+
+Status linrec_suffix(Context* ctx, const Fr* c, Fr* y, uint64_t n, const host::Fr4& k, cudaStream_t st,
+                     bool first_only = false) {
+    return linrec_suffix_batch(ctx, &c, &y, &k, 1, n, st, first_only);
 }
 
 // ---- permutation argument ----
@@ -553,20 +546,19 @@ Status logup_device(Context* ctx, const Domain* d, const mzk_logup_desc* desc, c
     }
     uint32_t total_cols = 0;
     for (uint32_t c = 0; c < desc->n_chunks; c++) total_cols += desc->chunk_cols[c];
-    void *tden_buf, *cols_buf, *ld_buf, *dbl;
-    MZK_TRY(ctx->ensure("logup_tden", (size_t)n * sizeof(Fr), &tden_buf));
-    MZK_TRY(ctx->ensure("logup_cols", (size_t)std::max(1u, total_cols) * n * sizeof(Fr), &cols_buf));
+    void *cols_buf, *ld_buf, *dbl;
+    // the table's column, then the inputs', inverted together
+    MZK_TRY(ctx->ensure("logup_cols", ((size_t)total_cols + 1) * n * sizeof(Fr), &cols_buf));
     MZK_TRY(ctx->ensure("logup_ld", (size_t)n * sizeof(Fr), &ld_buf));
     MZK_TRY(ctx->ensure("logup_blinds", ((size_t)bf + 1) * sizeof(Fr), &dbl));
     if (bf) MZK_CUDA_CHECK(cudaMemcpyAsync(dbl, desc->blinds, (size_t)bf * sizeof(Fr), cudaMemcpyHostToDevice, st));
-    Fr *tden = (Fr*)tden_buf, *cols = (Fr*)cols_buf, *ld = (Fr*)ld_buf;
+    Fr *tden = (Fr*)cols_buf, *cols = tden + n, *ld = (Fr*)ld_buf;
     const Fr beta = to_dev(to_host(desc->beta));
     const uint32_t grid = grid_for(ctx, n, kThreads);
-    // T = 1 / (t + beta)
+    // T = 1 / (t + beta) and, for every input column, 1 / (f + beta) (inverting
+    // them together gives the same field values)
     k_add_const<<<grid, kThreads, 0, st>>>(reinterpret_cast<const Fr*>(desc->table), beta, tden, n);
     MZK_LAUNCH_CHECK(ctx);
-    MZK_TRY(batch_invert(ctx, tden, n, st));
-    // every input column: 1 / (f + beta) (inverting them together gives the same field values)
     for (uint32_t j = 0; j < total_cols; j++) {
         if (!desc->inputs[j]) {
             set_error("logup: null input column");
@@ -576,7 +568,7 @@ Status logup_device(Context* ctx, const Domain* d, const mzk_logup_desc* desc, c
                                                cols + (size_t)j * n, n);
         MZK_LAUNCH_CHECK(ctx);
     }
-    MZK_TRY(batch_invert(ctx, cols, (uint64_t)total_cols * n, st));
+    MZK_TRY(batch_invert(ctx, tden, ((uint64_t)total_cols + 1) * n, st));
     HelperPtrs hp;
     hp.chunks = desc->n_chunks;
     for (uint32_t c = 0, j = 0; c < desc->n_chunks; j += desc->chunk_cols[c], c++) {
@@ -661,8 +653,8 @@ Status eval_polynomial_device(Context* ctx, const void* poly, uint64_t n, const 
     std::memset(out, 0, 32);
     if (n == 0) return OK;
     void* y;
-    MZK_TRY(ctx->ensure("grand_eval", n * sizeof(Fr), &y));
-    MZK_TRY(linrec_suffix(ctx, static_cast<const Fr*>(poly), (Fr*)y, n, to_host(point), st));
+    MZK_TRY(ctx->ensure("grand_eval", sizeof(Fr), &y));
+    MZK_TRY(linrec_suffix(ctx, static_cast<const Fr*>(poly), (Fr*)y, n, to_host(point), st, true));
     MZK_CUDA_CHECK(cudaMemcpyAsync(out, y, 32, cudaMemcpyDeviceToHost, st));
     MZK_CUDA_CHECK(cudaStreamSynchronize(st));
     return OK;
