@@ -714,14 +714,28 @@ __global__ void __launch_bounds__(kAccThreads) k_accumulate_quads(const Affine* 
 // chunks few chunks start one, and walking the chunks instead left most quads
 // idle (proof of 2^14 rows, six calls: 699 us).  A bucket spanning many chunks
 // (a heavy bucket: scalars 0/1, a nearly empty top window) is queued for
-// k_fixup_long, whose 64 quads take ~30 us for any span up to 65: the chain of
-// 12 additions that a quad still takes itself costs ~55.
+// k_fixup_pieces: the chain of 12 additions that a quad still takes itself costs
+// ~55 us, a block's tree ~30 for any span up to 64.
 constexpr uint32_t kShortSpan = 12;
 
+// Long spans in two steps: pieces of kPiece chunks, each one block's tree of
+// quads, whose sums take the place of the piece's first partial; then the
+// pieces of a span.  A span of 600 chunks (a column of small values in a proof
+// of 2^14 rows) is a chain of 6 + 4 additions instead of the 10 + 6 of a block
+// that strides over it.
+constexpr uint32_t kPiece = 64;
 struct LongSpans {
-    uint32_t* count;
-    uint4* list;  // (first chunk, last chunk, bucket key)
+    uint32_t* count;  // spans, pieces
+    uint4* list;      // (first chunk, last chunk, bucket key, -)
+    uint4* pieces;    // (first chunk of the span, piece, its last chunk, -)
 };
+__host__ __device__ constexpr uint32_t pieces_of(uint32_t first, uint32_t last) {
+    return (last - first) / kPiece + 1;
+}
+// where the sum of a span's piece lives
+__device__ __forceinline__ size_t piece_slot(uint32_t first, uint32_t piece) {
+    return 2 * ((size_t)first + (size_t)piece * kPiece) + (piece == 0 ? 1u : 0u);
+}
 
 __global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __restrict__ offsets, uint32_t keys,
                                                           uint32_t chunks, const Xyzz* __restrict__ partials,
@@ -739,7 +753,11 @@ __global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __rest
         last = (offsets[k + 1] - 1) / len;
         u = t + 1;
         if (last - t > kShortSpan) {
-            if ((threadIdx.x & 3) == 0) spans.list[atomicAdd(spans.count, 1u)] = make_uint4(t, last, k, 0);
+            if ((threadIdx.x & 3) == 0) {
+                spans.list[atomicAdd(spans.count, 1u)] = make_uint4(t, last, k, 0);
+                const uint32_t np = pieces_of(t, last), at = atomicAdd(spans.count + 1, np);
+                for (uint32_t p = 0; p < np; p++) spans.pieces[at + p] = make_uint4(t, p, last, 0);
+            }
             mine = false;
             last = t;
         } else {
@@ -751,30 +769,52 @@ __global__ void __launch_bounds__(kReduceThreads) k_fixup(const uint32_t* __rest
     if (mine) quad_store(&buckets[k], acc);
 }
 
-// one block per queued heavy bucket: its quads sum strided shares of the span,
-// then the block's points are added pairwise
-constexpr int kLongThreads = 256;
+constexpr int kLongThreads = 256;  // a quad per chunk of a piece
+static_assert(kLongThreads / 4 == kPiece, "one quad per chunk");
+
+// The quads' points added pairwise (warps stay together); the result in quad 0
+// and sm[0].  `live`: points beyond it are infinity.
+__device__ __forceinline__ void block_sum(Fp acc, Xyzz* sm, uint32_t live) {
+    const uint32_t quad = threadIdx.x >> 2;
+    quad_store(&sm[quad], acc);
+    __syncthreads();
+    uint32_t off = kPiece / 2;
+    while (off > 0 && off >= live) off >>= 1;
+    for (; off > 0; off >>= 1) {
+        if ((quad & ~7u) < off) {
+            const Fp r = quad_add(quad_load(&sm[quad]), quad < off ? quad_load(&sm[quad + off]) : fp_zero());
+            if (quad < off) quad_store(&sm[quad], r);
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(kLongThreads) k_fixup_pieces(Xyzz* __restrict__ partials, const LongSpans spans) {
+    __shared__ Xyzz sm[kPiece];
+    const uint32_t quad = threadIdx.x >> 2;
+    for (uint32_t i = blockIdx.x; i < spans.count[1]; i += gridDim.x) {
+        const uint4 pc = spans.pieces[i];
+        const uint32_t first = pc.x, piece = pc.y, last = pc.z;
+        const uint32_t u = first + piece * kPiece + quad;
+        const uint32_t live = min(kPiece, last - (first + piece * kPiece) + 1);
+        const Fp acc = quad < live ? quad_load(&partials[u == first ? 2 * (size_t)u + 1 : 2 * (size_t)u]) : fp_zero();
+        block_sum(acc, sm, live);
+        if (quad == 0) quad_store(&partials[piece_slot(first, piece)], quad_load(&sm[0]));
+        __syncthreads();
+    }
+}
 
 __global__ void __launch_bounds__(kLongThreads) k_fixup_long(const Xyzz* __restrict__ partials, const LongSpans spans,
                                                              Xyzz* __restrict__ buckets) {
-    constexpr uint32_t kQuads = kLongThreads / 4;
-    __shared__ Xyzz sm[kQuads];
+    __shared__ Xyzz sm[kPiece];
     const uint32_t quad = threadIdx.x >> 2;
-    for (uint32_t item = blockIdx.x; item < *spans.count; item += gridDim.x) {
+    for (uint32_t item = blockIdx.x; item < spans.count[0]; item += gridDim.x) {
         const uint4 sp = spans.list[item];
-        const uint32_t t = sp.x, last = sp.y;
-        Fp acc = quad == 0 ? quad_load(&partials[2 * (size_t)t + 1]) : fp_zero();
-        for (uint32_t u = t + 1 + quad; __any_sync(0xffffffffu, u <= last); u += kQuads)
-            acc = quad_add(acc, u <= last ? quad_load(&partials[2 * (size_t)u]) : fp_zero());
-        quad_store(&sm[quad], acc);
-        __syncthreads();
-        for (uint32_t off = kQuads / 2; off > 0; off >>= 1) {
-            if ((quad & ~7u) < off) {  // warps stay together
-                const Fp r = quad_add(quad_load(&sm[quad]), quad < off ? quad_load(&sm[quad + off]) : fp_zero());
-                if (quad < off) quad_store(&sm[quad], r);
-            }
-            __syncthreads();
-        }
+        const uint32_t np = pieces_of(sp.x, sp.y);
+        Fp acc = quad < np ? quad_load(&partials[piece_slot(sp.x, quad)]) : fp_zero();
+        for (uint32_t p = quad + kPiece; __any_sync(0xffffffffu, p < np); p += kPiece)
+            acc = quad_add(acc, p < np ? quad_load(&partials[piece_slot(sp.x, p)]) : fp_zero());
+        block_sum(acc, sm, np);
         if (quad == 0) quad_store(&buckets[sp.z], quad_load(&sm[0]));
         __syncthreads();
     }
@@ -1089,17 +1129,21 @@ uint32_t accumulate_quad_blocks(const Context* ctx, uint64_t entries) {
     return entries > kQuadEntries ? 0u : (uint32_t)ctx->num_sms * 2;
 }
 
-// The queues of an accumulation: both counters in 16 bytes, then the owners
-// and the long spans (at most one of each per chunk).
+// The queues of an accumulation: the counters (owners; spans, pieces) in 16
+// bytes, then the long spans, their pieces (a span has more than kShortSpan
+// chunks, a piece kPiece but for a span's last, and every chunk lies in one span
+// but for its last bucket's: less than one per chunk of either) and the owners
+// (at most one per chunk).
 struct Queues {
     Owners own;
     LongSpans spans;
 };
-constexpr size_t queue_bytes(size_t chunks) { return 16 + chunks * (sizeof(uint4) + sizeof(uint2)); }
+constexpr size_t queue_bytes(size_t chunks) { return 16 + chunks * (2 * sizeof(uint4) + sizeof(uint2)); }
 Queues queues_at(void* p, size_t chunks) {
     uint32_t* counts = static_cast<uint32_t*>(p);
     uint4* spans = reinterpret_cast<uint4*>(counts + 4);
-    return {{counts, reinterpret_cast<uint2*>(spans + chunks)}, {counts + 1, spans}};
+    uint4* pieces = spans + chunks;
+    return {{counts, reinterpret_cast<uint2*>(pieces + chunks)}, {counts + 1, spans, pieces}};
 }
 
 template <bool kHalves = false>
@@ -1154,6 +1198,7 @@ cudaError_t launch_fixup(const Accumulation& a, cudaStream_t st) {
     const uint32_t chunks = a.quad_blocks ? a.quad_blocks * (kAccThreads / 4) : a.acc_blocks * kAccThreads;
     k_fixup<<<chunks * 4 / kReduceThreads, kReduceThreads, 0, st>>>(a.offsets, a.keys, chunks, a.partials, q.own,
                                                                    a.buckets, q.spans);
+    k_fixup_pieces<<<a.long_blocks, kLongThreads, 0, st>>>(a.partials, q.spans);
     k_fixup_long<<<a.long_blocks, kLongThreads, 0, st>>>(a.partials, q.spans, a.buckets);
     return cudaGetLastError();
 }
@@ -1251,7 +1296,7 @@ Status accumulate(Context* ctx, const Accumulation& all, const std::vector<KeyRa
             MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
         }
         MZK_CUDA_CHECK(launch_fixup(a, st));
-        ctx->launches += 3;
+        ctx->launches += 4;
     }
     return ctx->phase_end(st);
 }
