@@ -1459,12 +1459,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
 
     // host: sum_w 2^(c w) S_w by Horner, then normalise
     const host::Xyzz6* hs = static_cast<const host::Xyzz6*>(host_wsum);
-    host::Xyzz6 acc = host::infinity();
-    for (int w = sh.windows - 1; w >= 0; w--) {
-        for (int b = 0; b < sh.c; b++) acc = host::dbl(acc);
-        acc = host::add(acc, host::canon(hs[w]));
-    }
-    host::to_jacobian_normalised(acc, out18);
+    host::combine_windows(hs, sh.windows, sh.c, out18);
     return OK;
 }
 
@@ -1725,16 +1720,9 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     std::vector<size_t> first_win(hi.size());
     for (size_t i = 0, w0 = 0; i < hi.size(); w0 += hi[i].fixed ? 1 : hi[i].windows, i++) first_win[i] = w0;
     auto tail = [&](size_t i) {
-        host::Xyzz6 acc = host::infinity();
-        if (hi[i].fixed) {  // the table rows already carry the 2^(c w) factors
-            acc = host::canon(hs[first_win[i]]);
-        } else {
-            for (int w = (int)hi[i].windows - 1; w >= 0; w--) {
-                for (uint32_t b = 0; b < hi[i].c; b++) acc = host::dbl(acc);
-                acc = host::add(acc, host::canon(hs[first_win[i] + w]));
-            }
-        }
-        host::to_jacobian_normalised(acc, out + 18 * item_of[i]);
+        // fixed: one window, the table rows already carry the 2^(c w) factors
+        host::combine_windows(hs + first_win[i], hi[i].fixed ? 1 : (int)hi[i].windows, (int)hi[i].c,
+                              out + 18 * item_of[i]);
     };
     const size_t cores = std::max(1u, std::thread::hardware_concurrency());
     const size_t nthreads = std::min<size_t>({hi.size() / 2, cores / 2, 32});
@@ -1910,12 +1898,7 @@ Status msm_g1_noalloc_queued(unsigned char* base, int sms, const void* d_scalars
     host::Xyzz6 hs[kNaMaxWindows];
     MZK_CUDA_CHECK(cudaMemcpyAsync(hs, wsum, (size_t)sh.windows * sizeof(Xyzz), cudaMemcpyDeviceToHost, st));
     MZK_CUDA_CHECK(cudaStreamSynchronize(st));
-    host::Xyzz6 acc = host::infinity();
-    for (int w = sh.windows - 1; w >= 0; w--) {
-        for (int b = 0; b < sh.c; b++) acc = host::dbl(acc);
-        acc = host::add(acc, host::canon(hs[w]));
-    }
-    host::to_jacobian_normalised(acc, out18);
+    host::combine_windows(hs, sh.windows, sh.c, out18);
     return OK;
 }
 
