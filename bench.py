@@ -41,7 +41,9 @@ sys.path.insert(0, str(ROOT))
 METRIC = "G1 MSM Mpts/s at 2^24"
 UNIT = "Mpts/s"
 IMAD_PER_FP_MUL = 600        # CIOS, 12 limbs: 2*12^2+12 = 300 products x (lo, hi)
-FP_MUL_PER_MIXED_ADD = 10    # madd-2008-s: 8M + 2S
+# per bucket entry at 2^24: three rounds of affine pair sums (7/8 of the entries, 5M + 1S
+# each, inversions left out), mixed additions (1/8, 8M + 2S)
+FP_MUL_PER_ENTRY = 6.5
 IMAD_PER_POINT_REF = 97.0e3  # reference schedule c=17, W=16 at 2^24: 1.628e12 IMAD / 2^24
 
 
@@ -130,7 +132,7 @@ class ClockSampler:
 
 
 def traffic_from_profiles(c):
-    """DRAM bytes per bucket entry of the accumulate kernel from the committed ncu summary."""
+    """DRAM bytes per bucket entry of the accumulation's kernels from the committed ncu summary."""
     f = ROOT / "profiles" / "msm_accumulate.md"
     if not f.exists():
         return None
@@ -767,17 +769,17 @@ def run_ours(args):
 
     acc_ms, acc_cnt = phases["accumulate"]
     acc_avg_ms = acc_ms / max(acc_cnt, 1)
-    imad_acc = entries * FP_MUL_PER_MIXED_ADD * IMAD_PER_FP_MUL
+    imad_acc = entries * FP_MUL_PER_ENTRY * IMAD_PER_FP_MUL
     achieved = imad_acc / (acc_avg_ms / 1e3)
     tpe = traffic_from_profiles(c)
     roofline = {
-        "kernel": "k_accumulate (bucket accumulation)", "bound": "imad",
+        "kernel": "k_pair_sums and k_accumulate (bucket accumulation)", "bound": "imad",
         "achieved": round(achieved / 1e12, 3), "peak": round(imad_peak / 1e12, 3), "unit": "TIMAD/s",
         "frac": round(achieved / imad_peak, 4),
         "traffic": None if tpe is None else round(tpe * entries),
         "peak_source": "measured in this run: max of mzk_probe_imad_peak's IMAD microbenchmarks and "
                        "600 x the measured 12-limb Montgomery multiplication rate (per-thread operands)",
-        "work": f"{entries} bucket entries x {FP_MUL_PER_MIXED_ADD} Fp mul x {IMAD_PER_FP_MUL} IMAD",
+        "work": f"{entries} bucket entries x {FP_MUL_PER_ENTRY} Fp mul x {IMAD_PER_FP_MUL} IMAD",
         "launch_ms": round(acc_avg_ms, 3),
     }
     msm_roof = {
