@@ -428,13 +428,14 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
 // products).  With ~40 products' worth of time for the inversion
 // (inv_divsteps) an addition costs ~7 products against the 10 of a mixed XYZZ
 // addition, at the price of writing the sums (96 bytes each) and reading them
-// again.  The multiply pipe is 70-72 % busy (88 % in k_accumulate): the rest
-// are waits for loads that one sum's lead does not cover and, with two warps
-// per scheduler, the latency of the products themselves.  1000003 points: 8.4 M
-// + 4.2 M + 2.1 M sums take 2.33 + 1.24 + 0.64 ms and leave 0.83 ms of mixed
-// additions, 5.8 ms without.  A third warp per scheduler spills (168
-// registers) and is slower (7.34 ms per call against 6.66), as are 48 sums per
-// inversion.
+// again.  The multiply pipe is ~70 % busy (88 % in k_accumulate): the rest are
+// waits for loads that one sum's lead does not cover, instruction fetch and, with
+// two warps per scheduler, the latency of the products themselves.  A third
+// warp spills (168 registers) and is slower; the x coordinates two sums ahead
+// are 1 % slower.  Per call with 64 / 96 / 128 / 256 sums per inversion: 1000003
+// points 6.61 / 6.62 / 6.32 / 6.17 ms, 2^24 points 87.1 / 85.7 / 84.0 / 82.0, eight
+// proofs of 2^16 rows 55.4 / 54.2 / 53.8 / 52.5 (7.34, 92.0 and 58.9 ms without
+// pair sums).
 //
 // A thread takes a run of consecutive sums: forward it multiplies up the
 // denominators and keeps the partial products, then inverts, then backward it
@@ -489,21 +490,43 @@ static __device__ __noinline__ PairCase pair_case(const Affine a, const Affine b
 }
 
 constexpr int kPairThreads = 128;
-constexpr int kPairBatch = 64;  // sums that share an inversion
+// Whether a + b may not be the chord's (d = x_b - x_a zero, a point at
+// infinity): by the first words, wrong in 2^30 for sums that are, which
+// pair_case then sorts out.
+__device__ __forceinline__ bool maybe_special(const Fp& d, const Fp& xa, const Fp& xb) {
+    return d.l[0] == 0u || d.l[0] == FpP::mod(0) || xa.l[0] == 0u || xb.l[0] == 0u;
+}
+
+constexpr int kPairBatch = 256;  // sums that share an inversion
+
+// What a thread keeps of its batch, element i of thread t at i * threads + t
+// (a partial product in three planes of 16 bytes), so that a warp's accesses
+// are contiguous: 56 bytes per sum, 543 MB for 37888 threads.
+struct PairScratch {
+    uint4* prefix;
+    uint32_t *ent1, *ent2;
+};
+constexpr size_t pair_scratch_bytes(size_t threads) { return threads * kPairBatch * (sizeof(Fp) + 2 * sizeof(uint32_t)); }
+PairScratch pair_scratch_at(void* p, size_t threads) {
+    uint4* prefix = static_cast<uint4*>(p);
+    uint32_t* ent = reinterpret_cast<uint32_t*>(prefix + 3 * threads * kPairBatch);
+    return {prefix, ent, ent + threads * kPairBatch};
+}
 
 // Sum j of bucket k: points off_in[k] + 2 (j - off_out[k]) and the next, if
 // that is below off_in[k + 1].  kGather: point i is src[sorted[i]] with the
 // entry's sign, otherwise src[i].
-template <int B, bool kGather>
+template <bool kGather>
 __global__ void __launch_bounds__(kPairThreads, 2) k_pair_sums(const Affine* __restrict__ src,
                                                                const uint32_t* __restrict__ sorted,
                                                                const uint32_t* __restrict__ off_in,
                                                                const uint32_t* __restrict__ off_out, uint32_t keys,
-                                                               Affine* __restrict__ out) {
-    static_assert(B <= 64, "a bit per sum");
+                                                               Affine* __restrict__ out, const PairScratch scratch) {
+    constexpr uint32_t B = kPairBatch;
+    const uint32_t threads = gridDim.x * blockDim.x;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t s, e;
-    chunk_range(off_out[keys], t, gridDim.x * blockDim.x, s, e);
+    chunk_range(off_out[keys], t, threads, s, e);
     if (s >= e) return;
     // the point of an entry: index | sign << 31 when gathering, else the index
     auto point = [&](uint32_t ent) { return load_affine(src, kGather ? ent & 0x7fffffffu : ent); };
@@ -515,11 +538,29 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_sums(const Affine* __r
     uint32_t k = find_key(off_out, keys, s);
     uint32_t lo = off_out[k], hi = off_out[k + 1], in_lo = off_in[k], in_hi = off_in[k + 1];
     const uint32_t rounds = (e - s + B - 1) / B, per = (e - s + rounds - 1) / rounds;
-    Fp prefix[B];
-    uint32_t ent1[B], ent2[B];
+    uint32_t* const ents1 = scratch.ent1 + t;
+    uint32_t* const ents2 = scratch.ent2 + t;
+    auto ent1 = [&](int i) -> uint32_t& { return ents1[(size_t)i * threads]; };
+    auto ent2 = [&](int i) -> uint32_t& { return ents2[(size_t)i * threads]; };
+    auto put_prefix = [&](int i, const Fp& v) {
+#pragma unroll
+        for (int p = 0; p < 3; p++)
+            scratch.prefix[((size_t)i * 3 + p) * threads + t] = make_uint4(v.l[4 * p], v.l[4 * p + 1], v.l[4 * p + 2], v.l[4 * p + 3]);
+    };
+    auto get_prefix = [&](int i) {
+        Fp v;
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            const uint4 q = scratch.prefix[((size_t)i * 3 + p) * threads + t];
+            v.l[4 * p] = q.x;
+            v.l[4 * p + 1] = q.y;
+            v.l[4 * p + 2] = q.z;
+            v.l[4 * p + 3] = q.w;
+        }
+        return v;
+    };
     for (uint32_t j0 = s; j0 < e; j0 += per) {
         const int n = (int)min(per, e - j0);
-        uint64_t pairs = 0, plain = 0;  // sum i adds two points; by the chord of two finite points
         for (int i = 0; i < n; i++) {
             const uint32_t j = j0 + (uint32_t)i;
             while (j >= hi) {
@@ -531,79 +572,78 @@ __global__ void __launch_bounds__(kPairThreads, 2) k_pair_sums(const Affine* __r
             }
             const uint32_t p = in_lo + 2 * (j - lo);
             const bool two = p + 1 < in_hi;
-            ent1[i] = kGather ? __ldg(sorted + p) : p;
-            ent2[i] = kGather ? (two ? __ldg(sorted + p + 1) : 0u) : p + 1;
-            if (two) pairs |= 1ull << i;
+            ent1(i) = kGather ? __ldg(sorted + p) : p;
+            ent2(i) = !two ? kNoKey : kGather ? __ldg(sorted + p + 1) : p + 1;
         }
         // forward: the x of the next sum's points are loaded one sum ahead and
         // its entries two, so that no address waits on a load
-        uint32_t c1 = ent1[0], c2 = ent2[0], e1 = 0, e2 = 0;
+        uint32_t c1 = ent1(0), c2 = ent2(0), e1 = 0, e2 = kNoKey;
         Fp acc = fp_one(), n1 = fp_zero(), n2 = fp_zero();
-        if (pairs & 1ull) {
+        if (c2 != kNoKey) {
             n1 = point_x(c1);
             n2 = point_x(c2);
         }
         if (n > 1) {
-            e1 = ent1[1];
-            e2 = ent2[1];
+            e1 = ent1(1);
+            e2 = ent2(1);
         }
         for (int i = 0; i < n; i++) {
             const Fp x1 = n1, x2 = n2;
             const uint32_t p1 = c1, p2 = c2;
             c1 = e1;
             c2 = e2;
+            e2 = kNoKey;
             if (i + 2 < n) {
-                e1 = ent1[i + 2];
-                e2 = ent2[i + 2];
+                e1 = ent1(i + 2);
+                e2 = ent2(i + 2);
             }
-            if (i + 1 < n && ((pairs >> (i + 1)) & 1ull)) {
+            if (c2 != kNoKey) {
                 n1 = point_x(c1);
                 n2 = point_x(c2);
             }
-            if (!((pairs >> i) & 1ull)) continue;
+            if (p2 == kNoKey) continue;
             Fp d = fp_sub(x2, x1);
-            if (fp_is_zero(d) || fp_is_zero_raw(x1) || fp_is_zero_raw(x2)) {  // rare, infinity among them
+            if (maybe_special(d, x1, x2)) {
                 const PairCase c = pair_case(signed_point(point(p1), p1), signed_point(point(p2), p2));
                 if (c.kind == kPairFirst || c.kind == kPairSecond || c.kind == kPairInfinity) continue;
                 d = c.den;
-            } else {
-                plain |= 1ull << i;
             }
-            prefix[i] = acc;
+            put_prefix(i, acc);
             acc = fp_mul(acc, d);
         }
         Fp inv = fp_invert(acc);
         // backward: points and partial product one sum ahead, entries two
-        c1 = ent1[n - 1];
-        c2 = ent2[n - 1];
+        c1 = ent1(n - 1);
+        c2 = ent2(n - 1);
         if (n > 1) {
-            e1 = ent1[n - 2];
-            e2 = ent2[n - 2];
+            e1 = ent1(n - 2);
+            e2 = ent2(n - 2);
         }
         Affine na = point(c1), nb = na;
-        Fp npre = prefix[n - 1];
-        if ((pairs >> (n - 1)) & 1ull) nb = point(c2);
+        Fp npre = get_prefix(n - 1);
+        if (c2 != kNoKey) nb = point(c2);
         for (int i = n - 1; i >= 0; i--) {
             Affine a = signed_point(na, c1);
             const Affine b = signed_point(nb, c2);
             const Fp pre = npre;
+            const bool two = c2 != kNoKey;
             c1 = e1;
             c2 = e2;
             if (i > 1) {
-                e1 = ent1[i - 2];
-                e2 = ent2[i - 2];
+                e1 = ent1(i - 2);
+                e2 = ent2(i - 2);
             }
             if (i > 0) {
                 na = point(c1);
-                if ((pairs >> (i - 1)) & 1ull) {
+                if (c2 != kNoKey) {
                     nb = point(c2);
-                    npre = prefix[i - 1];
+                    npre = get_prefix(i - 1);
                 }
             }
-            if ((pairs >> i) & 1ull) {
+            if (two) {
                 Fp d = fp_sub(b.x, a.x), num = fp_sub(b.y, a.y);
                 int kind = kPairAdd;
-                if (!((plain >> i) & 1ull)) {
+                if (maybe_special(d, a.x, b.x)) {  // as in the forward pass
                     const PairCase c = pair_case(a, b);
                     kind = c.kind;
                     d = c.den;
@@ -1212,7 +1252,8 @@ struct KeyRange {
 // Rounds of pair sums for `entries` entries over `keys` buckets.  A sum costs
 // less than a mixed addition only while a thread has ~48 to share an inversion
 // (the lanes' grid has 37888 threads), and a round halves buckets of four
-// points or more.  Per call without / with 1 / 2 / 3 rounds: 1000003 points (16.8
+// points or more.  Per call without / with 1 / 2 / 3 rounds, 64 sums per
+// inversion: 1000003 points (16.8
 // M entries, 32 per bucket) 7.34 / 6.86 / 6.73 / 6.66 ms, 4000000 points 25.4 /
 // 23.5 / 22.6 / 22.2, 2^24 points 92.0 / 90.0 / 88.0 / 87.4; 262144 points (5 M
 // entries) 2.60 / 2.59 / 2.59 / 2.62.
@@ -1261,18 +1302,24 @@ Status accumulate(Context* ctx, const Accumulation& all, const std::vector<KeyRa
     }
     void *sums[2] = {}, *offs[2] = {};
     bool paired = rounds > 0;
+    uint32_t blocks = 0;
+    PairScratch scratch{};
     if (paired) {
+        int per_sm = 0;
+        MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_sums<true>, kPairThreads, 0));
+        blocks = (uint32_t)ctx->num_sms * (uint32_t)std::max(1, per_sm);
+        const size_t threads = (size_t)blocks * kPairThreads;
+        void* mem = nullptr;
         const uint64_t cap0 = (most + most_keys) / 2 + 1, cap1 = (cap0 + most_keys) / 2 + 1;
-        paired = ctx->ensure("msm_sums0", cap0 * sizeof(Affine), &sums[0]) == OK &&
+        paired = ctx->ensure("msm_pair_scratch", pair_scratch_bytes(threads), &mem) == OK &&
+                 ctx->ensure("msm_sums0", cap0 * sizeof(Affine), &sums[0]) == OK &&
                  (rounds < 2 || ctx->ensure("msm_sums1", cap1 * sizeof(Affine), &sums[1]) == OK) &&
                  ctx->ensure("msm_sum_off0", (most_keys + 2) * 4, &offs[0]) == OK &&
                  (rounds < 2 || ctx->ensure("msm_sum_off1", (most_keys + 2) * 4, &offs[1]) == OK);
+        if (paired) scratch = pair_scratch_at(mem, threads);
     }
     MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
     if (!paired) parts.assign(1, {0, all.keys, entries});
-    int per_sm = 0;
-    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_sums<kPairBatch, true>, kPairThreads, 0));
-    const uint32_t blocks = (uint32_t)ctx->num_sms * (uint32_t)std::max(1, per_sm);
     for (const Part& p : parts) {
         Accumulation a = all;
         a.keys = p.k1 - p.k0;
@@ -1283,9 +1330,9 @@ Status accumulate(Context* ctx, const Accumulation& all, const std::vector<KeyRa
             Affine* out = static_cast<Affine*>(sums[r & 1]);
             MZK_TRY(scan_u32<true>(ctx, a.offsets, off, a.keys + 1, st));
             if (r == 0)
-                k_pair_sums<kPairBatch, true><<<blocks, kPairThreads, 0, st>>>(a.bases, a.sorted, a.offsets, off, a.keys, out);
+                k_pair_sums<true><<<blocks, kPairThreads, 0, st>>>(a.bases, a.sorted, a.offsets, off, a.keys, out, scratch);
             else
-                k_pair_sums<kPairBatch, false><<<blocks, kPairThreads, 0, st>>>(a.bases, nullptr, a.offsets, off, a.keys, out);
+                k_pair_sums<false><<<blocks, kPairThreads, 0, st>>>(a.bases, nullptr, a.offsets, off, a.keys, out, scratch);
             MZK_LAUNCH_CHECK(ctx);
             a.offsets = off;
             a.bases = out;
