@@ -189,6 +189,14 @@ int mzk_msm_set_window(mzk_ctx *ctx, int c);
 int mzk_msm_pick_window(size_t n);
 /* Window width, window count and bucket entries (non-zero digits) of the last MSM. */
 int mzk_msm_last_shape(mzk_ctx *ctx, int *c, int *windows, uint64_t *entries);
+/* Device memory that large MSMs of this context may hold to add the points of a
+ * bucket in pairs first (default 3.125 GiB; below ~0.6 GB, or where it is not to be
+ * had, they run without, more slowly, with the same results).  Memory held
+ * beyond the new limit is freed at once; 0 frees all of it. */
+int mzk_msm_set_pair_memory(mzk_ctx *ctx, uint64_t bytes);
+/* Rounds of pair sums that the last MSM took (0: none), and the parts its buckets were
+ * cut into for that memory (a pipelined host MSM: of its last upload part). */
+int mzk_msm_last_pair_sums(mzk_ctx *ctx, int *rounds, int *parts);
 
 /* ---- EvaluationDomain (proofs/src/poly/domain.rs) ----------------------- */
 typedef struct mzk_domain mzk_domain;

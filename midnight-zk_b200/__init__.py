@@ -74,6 +74,8 @@ SIGNATURES = {
     "mzk_msm_g1_noalloc": (_i32, [_vp, _vp, _sz, _u64p, _vp]),
     "mzk_msm_g1_batch_device": (_i32, [_vp, _vp, _sz, _vp, _sz, _u64p]),
     "mzk_msm_set_window": (_i32, [_vp, _i32]),
+    "mzk_msm_set_pair_memory": (_i32, [_vp, _u64]),
+    "mzk_msm_last_pair_sums": (_i32, [_vp, ctypes.POINTER(_i32), ctypes.POINTER(_i32)]),
     "mzk_msm_pick_window": (_i32, [_sz]),
     "mzk_domain_create": (_i32, [_vp, _u32, _u32, ctypes.POINTER(_vp)]),
     "mzk_domain_destroy": (_i32, [_vp]),
@@ -570,7 +572,17 @@ class Context:
         _check(lib().mzk_msm_last_shape(self.h, ctypes.byref(c), ctypes.byref(w), _ptr(e)))
         return c.value, w.value, int(e[0])
 
+    def msm_last_pair_sums(self):
+        """(rounds, parts) of the last MSM's pair sums."""
+        r, p = _i32(), _i32()
+        _check(lib().mzk_msm_last_pair_sums(self.h, ctypes.byref(r), ctypes.byref(p)))
+        return r.value, p.value
+
     # ---- MSM ----
+    def set_msm_pair_memory(self, nbytes):
+        """Device memory this context's large MSMs may hold for their pair sums (0: none)."""
+        _check(lib().mzk_msm_set_pair_memory(self.h, int(nbytes)))
+
     def set_msm_window(self, c):
         _check(lib().mzk_msm_set_window(self.h, int(c)))
 

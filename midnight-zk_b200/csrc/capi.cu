@@ -81,6 +81,28 @@ Status Context::ensure_pinned(size_t bytes, void** out) {
     return OK;
 }
 
+void* Context::pair_memory(size_t bytes) {
+    if (pair.bytes >= bytes) return pair.p;
+    const bool grown = pair.p != nullptr;
+    pair_release();
+    if (bytes > pair_limit) return nullptr;
+    if (grown) bytes = std::min<uint64_t>(bytes + bytes / 4, pair_limit);  // as in ensure()
+    if (cudaMalloc(&pair.p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        pair.p = nullptr;
+        return nullptr;
+    }
+    pair.bytes = bytes;
+    return pair.p;
+}
+
+void Context::pair_release() {
+    if (!pair.p) return;
+    cudaStreamSynchronize(stream);  // queued MSMs may still use it
+    cudaFree(pair.p);
+    pair = DevBuf{};
+}
+
 Status Context::phase_begin(int phase, cudaStream_t st) {
     if (!profiling) return OK;
     if (prof_used >= kMaxRecords) {
@@ -120,6 +142,7 @@ Context::~Context() {
     for (auto& kv : bufs)
         if (kv.second.p) cudaFree(kv.second.p);
     if (pinned) cudaFreeHost(pinned);
+    if (pair.p) cudaFree(pair.p);
     if (gen_table) cudaFree(gen_table);
     for (cudaEvent_t ev : ev_copy)
         if (ev) cudaEventDestroy(ev);
@@ -270,6 +293,22 @@ int mzk_msm_set_window(mzk_ctx* ctx, int c) {
     }
     Guard g(ctx);
     ctx->impl.msm_window_override = c;
+    return mzk::OK;
+}
+
+int mzk_msm_set_pair_memory(mzk_ctx* ctx, uint64_t bytes) {
+    if (int s = check_ctx(ctx)) return s;
+    Guard g(ctx);
+    ctx->impl.pair_limit = bytes;
+    if (ctx->impl.pair.bytes > bytes) ctx->impl.pair_release();
+    return mzk::OK;
+}
+
+int mzk_msm_last_pair_sums(mzk_ctx* ctx, int* rounds, int* parts) {
+    if (int s = check_ctx(ctx)) return s;
+    Guard g(ctx);
+    if (rounds) *rounds = ctx->impl.last_pair_rounds;
+    if (parts) *parts = ctx->impl.last_pair_parts;
     return mzk::OK;
 }
 

@@ -1243,12 +1243,6 @@ cudaError_t launch_fixup(const Accumulation& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Consecutive keys and the most entries they can hold
-struct KeyRange {
-    uint32_t key_end;
-    uint64_t entries;
-};
-
 // Rounds of pair sums for `entries` entries over `keys` buckets.  A sum costs
 // less than a mixed addition only while a thread has ~48 to share an inversion
 // (the lanes' grid has 37888 threads), and a round halves buckets of four
@@ -1266,78 +1260,185 @@ int pair_rounds(uint64_t entries, uint64_t keys) {
     return r;
 }
 
-// The bucket sums of all keys, by rounds of pair sums first where they pay.
-// The sums are formed for a part of the keys at a time (whole ranges, up to
-// kPairEntries entries), so that their arrays stay a few GB at any size.
-// Without memory for them the entries are accumulated as they are.  `entries`
-// is an upper bound (no zero digits); where it may call for rounds the true
-// number, which decides, is read back through `total` (pinned).
-constexpr uint64_t kPairEntries = 1u << 25;
+// ---- memory of the pair sums ----
+//
+// A context holds at most pair_limit bytes for them, whatever the call: the
+// scratch of k_pair_sums, and for one part of the keys at a time two arrays of
+// sums and two of offsets.  The parts are cut by the true counts (k_part_keys),
+// not by the callers' items or windows, since one bucket set may hold every
+// entry of a call (an item over a window table).  Where a single bucket and its
+// neighbours exceed the room their entries are accumulated as they are.
+constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-Status accumulate(Context* ctx, const Accumulation& all, const std::vector<KeyRange>& ranges, uint64_t entries,
-                  uint32_t* total, cudaStream_t st) {
-    int rounds = all.quad_blocks ? 0 : pair_rounds(entries, all.keys);
-    if (rounds) {
-        MZK_CUDA_CHECK(cudaMemcpyAsync(total, all.offsets + all.keys, 4, cudaMemcpyDeviceToHost, st));
-        MZK_CUDA_CHECK(cudaStreamSynchronize(st));
-        rounds = pair_rounds(*total, all.keys);
+// Where a part's arrays lie behind the scratch.  A round leaves at most half of
+// its points and one more per bucket.
+struct PairLayout {
+    size_t sums[2], offs[2], bytes;
+};
+PairLayout pair_layout(uint64_t entries, uint64_t keys, int rounds) {
+    const uint64_t n0 = std::min(entries, (entries + keys) / 2), n1 = std::min(n0, (n0 + keys) / 2);
+    PairLayout l;
+    l.offs[0] = 0;
+    l.offs[1] = l.offs[0] + align256((keys + 2) * 4);
+    l.sums[0] = l.offs[1] + (rounds > 1 ? align256((keys + 2) * 4) : 0);
+    l.sums[1] = l.sums[0] + align256((size_t)n0 * sizeof(Affine));
+    l.bytes = l.sums[1] + (rounds > 1 ? align256((size_t)n1 * sizeof(Affine)) : 0);
+    return l;
+}
+// bytes of a part are below this much per entry and key (entries = keys = half of both)
+constexpr uint64_t kPairBytes = sizeof(Affine) + 2 * sizeof(uint32_t);
+
+// Consecutive keys whose sums are formed together
+struct PairPart {
+    uint32_t k0, k1;   // keys
+    uint32_t first;    // offset of k0
+    uint64_t entries;
+    bool paired;       // false: accumulated as they are
+};
+
+// Split points i * step (i < n) of offset + key: the largest key at or below,
+// and its offset
+__global__ void k_part_keys(const uint32_t* __restrict__ offsets, uint32_t keys, uint64_t step, uint32_t n,
+                            uint2* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint64_t target = i * step;
+    uint32_t lo = 0, hi = keys + 1;
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if ((uint64_t)offsets[mid] + mid <= target) lo = mid;
+        else hi = mid;
     }
-    struct Part {
-        uint32_t k0, k1;
-        uint64_t entries;
+    out[i] = make_uint2(lo, offsets[lo]);
+}
+
+// A part's offsets from zero
+__global__ void k_rebase(const uint32_t* __restrict__ in, uint32_t len, uint32_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < len) out[i] = in[i] - in[0];
+}
+
+// Neighbouring split points joined into parts of at most `room` bytes, as few
+// as possible.  Empty where not even the offsets of one fit.
+std::vector<PairPart> join_greedily(const std::vector<uint2>& points, int rounds, uint64_t room) {
+    auto fits = [&](const uint2& a, const uint2& b) {
+        return pair_layout(b.y - a.y, b.x - a.x, rounds).bytes <= room;
     };
-    std::vector<Part> parts;
-    uint64_t most = 0, most_keys = 0;
-    if (rounds) {
-        uint32_t k = 0;
-        for (const KeyRange& r : ranges) {
-            if (parts.empty() || parts.back().entries + r.entries > kPairEntries) parts.push_back({k, k, 0});
-            parts.back().k1 = k = r.key_end;
-            parts.back().entries += r.entries;
-        }
-        for (const Part& p : parts) {
-            most = std::max(most, p.entries);
-            most_keys = std::max<uint64_t>(most_keys, p.k1 - p.k0);
-        }
+    std::vector<PairPart> parts;
+    for (size_t i = 0; i + 1 < points.size();) {
+        size_t j = i + 1;
+        while (j + 1 < points.size() && fits(points[i], points[j + 1])) j++;
+        const uint2 a = points[i], b = points[j];
+        i = j;
+        if (a.x == b.x) continue;
+        const PairPart p{a.x, b.x, a.y, b.y - a.y, fits(a, b)};
+        if (!p.paired && align256((size_t)(p.k1 - p.k0 + 2) * 4) > room) return {};
+        parts.push_back(p);
     }
-    void *sums[2] = {}, *offs[2] = {};
-    bool paired = rounds > 0;
-    uint32_t blocks = 0;
-    PairScratch scratch{};
-    if (paired) {
-        int per_sm = 0;
-        MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_sums<true>, kPairThreads, 0));
-        blocks = (uint32_t)ctx->num_sms * (uint32_t)std::max(1, per_sm);
-        const size_t threads = (size_t)blocks * kPairThreads;
-        void* mem = nullptr;
-        const uint64_t cap0 = (most + most_keys) / 2 + 1, cap1 = (cap0 + most_keys) / 2 + 1;
-        paired = ctx->ensure("msm_pair_scratch", pair_scratch_bytes(threads), &mem) == OK &&
-                 ctx->ensure("msm_sums0", cap0 * sizeof(Affine), &sums[0]) == OK &&
-                 (rounds < 2 || ctx->ensure("msm_sums1", cap1 * sizeof(Affine), &sums[1]) == OK) &&
-                 ctx->ensure("msm_sum_off0", (most_keys + 2) * 4, &offs[0]) == OK &&
-                 (rounds < 2 || ctx->ensure("msm_sum_off1", (most_keys + 2) * 4, &offs[1]) == OK);
-        if (paired) scratch = pair_scratch_at(mem, threads);
+    return parts;
+}
+
+// The split points of a call are at most 1 / kPairSteps of a part apart (more
+// only where they would be too many).
+constexpr uint32_t kPairSteps = 64, kMaxSplitPoints = 4096;
+
+// The same with parts of about equal size: a thread forms its share of a part in
+// batches of up to kPairBatch sums, and parts just over a multiple of that have
+// many small batches (2^24 points: 83.5 ms per call in full parts and a
+// remainder, 82.0 in equal ones; in windows, two at a time, 81.8).
+std::vector<PairPart> join_parts(const std::vector<uint2>& points, int rounds, uint64_t room) {
+    std::vector<PairPart> parts = join_greedily(points, rounds, room);
+    if (parts.size() < 2) return parts;
+    const uint64_t n = parts.size();
+    const uint64_t even = pair_layout(points.back().y / n, points.back().x / n, rounds).bytes;
+    std::vector<PairPart> evened = join_greedily(points, rounds, std::min(room, even + room / kPairSteps));
+    return evened.size() == n ? evened : parts;
+}
+
+// Rounds and parts of a call's pair sums (no parts: none).  `entries` is an
+// upper bound (no zero digits); where it calls for rounds the true number,
+// which decides, is read back through `total` (pinned), with the split points
+// where the call may not fit one part.
+Status plan_pairs(Context* ctx, const Accumulation& all, uint64_t entries, uint64_t room, uint32_t* total,
+                  int* rounds, std::vector<PairPart>* parts, cudaStream_t st) {
+    *rounds = all.quad_blocks ? 0 : pair_rounds(entries, all.keys);
+    if (!*rounds || !room) return OK;
+    std::vector<uint2> points;
+    if (pair_layout(entries, all.keys, *rounds).bytes > room) {
+        const uint64_t cost = entries + all.keys;
+        const uint64_t step = std::max(room / (kPairSteps * kPairBytes), cost / kMaxSplitPoints) + 1;
+        points.resize(cost / step + 1);
+        const uint32_t n = (uint32_t)points.size();
+        void* d;
+        MZK_TRY(ctx->ensure("msm_split_points", n * sizeof(uint2), &d));
+        k_part_keys<<<(n + 127) / 128, 128, 0, st>>>(all.offsets, all.keys, step, n, static_cast<uint2*>(d));
+        MZK_LAUNCH_CHECK(ctx);
+        MZK_CUDA_CHECK(cudaMemcpyAsync(points.data(), d, n * sizeof(uint2), cudaMemcpyDeviceToHost, st));
+    } else {
+        points.push_back(make_uint2(0, 0));
     }
+    MZK_CUDA_CHECK(cudaMemcpyAsync(total, all.offsets + all.keys, 4, cudaMemcpyDeviceToHost, st));
+    MZK_CUDA_CHECK(cudaStreamSynchronize(st));
+    points.push_back(make_uint2(all.keys, *total));
+    *rounds = pair_rounds(*total, all.keys);
+    if (*rounds) *parts = join_parts(points, *rounds, room);
+    return OK;
+}
+
+// The bucket sums of all keys, by rounds of pair sums first where they pay and
+// there is memory for them; the same results without.
+Status accumulate(Context* ctx, const Accumulation& all, uint64_t entries, uint32_t* total, cudaStream_t st) {
+    int per_sm = 0;
+    MZK_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pair_sums<true>, kPairThreads, 0));
+    const uint32_t blocks = (uint32_t)ctx->num_sms * (uint32_t)std::max(1, per_sm);
+    const size_t threads = (size_t)blocks * kPairThreads, fixed = align256(pair_scratch_bytes(threads));
+    int rounds = 0;
+    std::vector<PairPart> parts;
+    MZK_TRY(plan_pairs(ctx, all, entries, ctx->pair_limit > fixed ? ctx->pair_limit - fixed : 0, total, &rounds,
+                       &parts, st));
+    size_t need = 0;
+    for (const PairPart& p : parts)
+        need = std::max(need, p.paired ? pair_layout(p.entries, p.k1 - p.k0, rounds).bytes
+                                       : align256((size_t)(p.k1 - p.k0 + 2) * 4));
+    char* mem = nullptr;
+    if (!parts.empty()) mem = static_cast<char*>(ctx->pair_memory(fixed + need));
+    if (!mem) {
+        rounds = 0;
+        parts.assign(1, {0, all.keys, 0, entries, false});
+    }
+    ctx->last_pair_rounds = rounds;
+    ctx->last_pair_parts = mem ? (int)parts.size() : 0;
+    const PairScratch scratch = mem ? pair_scratch_at(mem, threads) : PairScratch{};
     MZK_TRY(ctx->phase_begin(PH_ACCUMULATE, st));
-    if (!paired) parts.assign(1, {0, all.keys, entries});
-    for (const Part& p : parts) {
+    for (const PairPart& p : parts) {
         Accumulation a = all;
         a.keys = p.k1 - p.k0;
         a.buckets = all.buckets + p.k0;
         a.offsets = all.offsets + p.k0;
-        for (int r = 0; paired && r < rounds; r++) {
-            uint32_t* off = static_cast<uint32_t*>(offs[r & 1]);
-            Affine* out = static_cast<Affine*>(sums[r & 1]);
-            MZK_TRY(scan_u32<true>(ctx, a.offsets, off, a.keys + 1, st));
-            if (r == 0)
-                k_pair_sums<true><<<blocks, kPairThreads, 0, st>>>(a.bases, a.sorted, a.offsets, off, a.keys, out, scratch);
-            else
-                k_pair_sums<false><<<blocks, kPairThreads, 0, st>>>(a.bases, nullptr, a.offsets, off, a.keys, out, scratch);
+        if (p.paired) {
+            const PairLayout l = pair_layout(p.entries, a.keys, rounds);
+            for (int r = 0; r < rounds; r++) {
+                uint32_t* off = reinterpret_cast<uint32_t*>(mem + fixed + l.offs[r & 1]);
+                Affine* out = reinterpret_cast<Affine*>(mem + fixed + l.sums[r & 1]);
+                MZK_TRY(scan_u32<true>(ctx, a.offsets, off, a.keys + 1, st));
+                if (r == 0)
+                    k_pair_sums<true><<<blocks, kPairThreads, 0, st>>>(a.bases, a.sorted, a.offsets, off, a.keys, out,
+                                                                       scratch);
+                else
+                    k_pair_sums<false><<<blocks, kPairThreads, 0, st>>>(a.bases, nullptr, a.offsets, off, a.keys, out,
+                                                                        scratch);
+                MZK_LAUNCH_CHECK(ctx);
+                a.offsets = off;
+                a.bases = out;
+            }
+        } else if (mem) {
+            uint32_t* off = reinterpret_cast<uint32_t*>(mem + fixed);
+            k_rebase<<<(a.keys + 1 + 255) / 256, 256, 0, st>>>(a.offsets, a.keys + 1, off);
             MZK_LAUNCH_CHECK(ctx);
             a.offsets = off;
-            a.bases = out;
+            a.sorted = all.sorted + p.first;
         }
-        MZK_CUDA_CHECK(launch_accumulate(a, !paired, st));
+        MZK_CUDA_CHECK(launch_accumulate(a, !p.paired, st));
         if (&p == &parts.back()) {  // one phase each per call, whatever the parts
             MZK_TRY(ctx->phase_end(st));
             MZK_TRY(ctx->phase_begin(PH_FIXUP, st));
@@ -1482,9 +1583,7 @@ Status msm_g1_parts(Context* ctx, const void* d_scalars, const void* d_bases, si
         if (part.bases_ready) MZK_CUDA_CHECK(cudaStreamWaitEvent(st, part.bases_ready, 0));
         const Accumulation acc{ba + part.begin, (const uint32_t*)sorted, off, sh.keys, (Xyzz*)buckets[p],
                                (Xyzz*)partials, queue, acc_blocks, quad_blocks, (uint32_t)ctx->num_sms * 2};
-        std::vector<KeyRange> ranges;
-        for (int w = 0; w < sh.windows; w++) ranges.push_back({(uint32_t)(w + 1) * sh.nb, np});
-        MZK_TRY(accumulate(ctx, acc, ranges, (uint64_t)sh.windows * np, host_entries + p, st));
+        MZK_TRY(accumulate(ctx, acc, (uint64_t)sh.windows * np, host_entries + p, st));
         MZK_CUDA_CHECK(cudaMemcpyAsync(host_entries + p, off + sh.keys, 4, cudaMemcpyDeviceToHost, st));
     }
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
@@ -1748,11 +1847,7 @@ Status msm_g1_batch_device(Context* ctx, const void* d_bases, size_t bases_len, 
     const Accumulation acc{static_cast<const Affine*>(d_bases), (const uint32_t*)sorted, (const uint32_t*)offsets,
                            (uint32_t)keys, (Xyzz*)buckets, (Xyzz*)partials, queue, acc_blocks, quad_blocks,
                            (uint32_t)ctx->num_sms * 2};
-    std::vector<KeyRange> ranges;
-    for (const BatchItemDev& it : hi)
-        for (uint32_t w = 0; w < (it.fixed ? 1u : it.windows); w++)
-            ranges.push_back({it.key_start + (w + 1) * it.nb, (uint64_t)it.n * (it.fixed ? it.windows : 1u)});
-    MZK_TRY(accumulate(ctx, acc, ranges, entries, static_cast<uint32_t*>(host_wsum), st));
+    MZK_TRY(accumulate(ctx, acc, entries, static_cast<uint32_t*>(host_wsum), st));
     MZK_TRY(ctx->phase_begin(PH_REDUCE, st));
     const BucketSets sets{{(const Xyzz*)buckets}, {(const uint32_t*)offsets}, 1};
     MZK_CUDA_CHECK(launch_reduce(plan, sets, d_tab, (Xyzz*)arena, (Xyzz*)wsum, &ctx->launches, st));
@@ -1812,7 +1907,6 @@ constexpr int kNoAllocMinC = 8, kNoAllocMaxC = 12;
 constexpr uint32_t kNoAllocAccBlocks = 64;  // fixed accumulate grid (64 x 128 threads)
 constexpr int kNoAllocMaxDevices = 64;
 
-constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // largest key count over the allowed widths: c = 12 gives 22 windows x 2048
 constexpr size_t kNaKeys = 22 * 2048;
 constexpr size_t kNaMaxWindows = 32;  // c = 8

@@ -45,6 +45,13 @@ struct Context {
     void* pinned = nullptr;
     size_t pinned_bytes = 0;
     int msm_window_override = 0;
+    // The pair sums of large MSMs (msm.cu) work in one optional buffer of at
+    // most pair_limit bytes; MSMs run without them where it is not to be had.
+    // The default (3.125 GiB) holds the sums of ~37 million bucket entries at a
+    // time, two full batches for every thread.
+    static constexpr uint64_t kPairLimit = 25ull << 27;
+    uint64_t pair_limit = kPairLimit;
+    DevBuf pair;
     // autotuned choices by floor(log2 size), 0 = not tuned (tune.cu): MSM
     // window width, NTT pass split (NttSplit, ntt.hpp)
     static constexpr int kTuneSlotsN = 33;
@@ -86,6 +93,7 @@ struct Context {
     // shape of the last MSM: window width, windows, bucket entries processed
     int last_c = 0, last_windows = 0;
     uint64_t last_entries = 0;
+    int last_pair_rounds = 0, last_pair_parts = 0;  // rounds of pair sums and parts of the keys
 
     // open/close a timed phase on `st` (no-ops unless profiling)
     Status phase_begin(int phase, cudaStream_t st);
@@ -96,6 +104,9 @@ struct Context {
     // device buffer `name` of at least `bytes` bytes (contents undefined)
     Status ensure(const char* name, size_t bytes, void** out);
     Status ensure_pinned(size_t bytes, void** out);
+    // the pair sums' buffer, of at least `bytes` bytes; null where it cannot be had
+    void* pair_memory(size_t bytes);
+    void pair_release();
     ~Context();
 };
 
