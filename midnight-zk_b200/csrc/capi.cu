@@ -51,7 +51,7 @@ Status Context::ensure(const char* name, size_t bytes, void** out) {
         bytes += bytes / 4;
     }
     bytes = (bytes + 255) & ~(size_t)255;
-    cudaError_t e = cudaMalloc(&b.p, bytes);
+    cudaError_t e = alloc(&b.p, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         b.p = nullptr;
@@ -81,12 +81,30 @@ Status Context::ensure_pinned(size_t bytes, void** out) {
     return OK;
 }
 
+cudaError_t Context::alloc(void** out, size_t bytes) {
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation && pair.p) {
+        cudaGetLastError();
+        pair_release();
+        e = cudaMalloc(out, bytes);
+    }
+    return e;
+}
+
 void* Context::pair_memory(size_t bytes) {
     if (pair.bytes >= bytes) return pair.p;
-    const bool grown = pair.p != nullptr;
+    // The buffer is optional and stays until it is released, so it takes at most
+    // a quarter of what is free: other contexts and allocators of the process
+    // cannot ask for it back as alloc() does.
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const uint64_t most = std::min<uint64_t>(pair_limit, (free_bytes + pair.bytes) / 4);
+    if (bytes > most) return nullptr;
+    if (pair.p) bytes = std::min<uint64_t>(bytes + bytes / 4, most);  // headroom as in ensure()
     pair_release();
-    if (bytes > pair_limit) return nullptr;
-    if (grown) bytes = std::min<uint64_t>(bytes + bytes / 4, pair_limit);  // as in ensure()
     if (cudaMalloc(&pair.p, bytes) != cudaSuccess) {
         cudaGetLastError();
         pair.p = nullptr;
@@ -257,7 +275,9 @@ int mzk_device_alloc(mzk_ctx* ctx, size_t bytes, void** out) {
     if (int s = check_ctx(ctx)) return s;
     if (!out) return mzk::ERR_ARG;
     Guard g(ctx);
-    MZK_CUDA_CHECK(cudaMalloc(out, bytes ? bytes : 16));
+    const cudaError_t e = ctx->impl.alloc(out, bytes ? bytes : 16);
+    if (e != cudaSuccess) cudaGetLastError();  // the next launch check would report it again
+    MZK_CUDA_CHECK(e);
     return mzk::OK;
 }
 

@@ -122,7 +122,7 @@ Status ensure_gen_table(Context* ctx) {
         for (int b = 0; b < 8; b++) base = host::dbl(base);
     }
     void* d;
-    MZK_CUDA_CHECK(cudaMalloc(&d, table.size() * 8));
+    MZK_CUDA_CHECK(ctx->alloc(&d, table.size() * 8));
     MZK_CUDA_CHECK(cudaMemcpy(d, table.data(), table.size() * 8, cudaMemcpyHostToDevice));
     ctx->gen_table = d;
     return OK;

@@ -347,11 +347,12 @@ static const Fr* pass_twiddles(Context* ctx, const Domain* d, int root, uint32_t
     if (it != d->pass_tw.end()) return it->second;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return nullptr;
-    Fr* p = nullptr;
-    if (cudaMalloc(&p, ((size_t)1 << log_s) * sizeof(Fr)) != cudaSuccess) {
+    void* mem = nullptr;
+    if (ctx->alloc(&mem, ((size_t)1 << log_s) * sizeof(Fr)) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
+    Fr* p = static_cast<Fr*>(mem);
     k_pass_twiddles<<<grid_for(ctx, 1u << log_s, 256), 256, 0, st>>>(d->lo[root], d->hi[root], log_n, log_s, log_r, p);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
         cudaFree(p);
@@ -422,13 +423,15 @@ Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
         const uint32_t N = 1u << logs[r];
         const uint32_t lo = std::min<uint32_t>(N, 1u << kLoBits);
         const uint32_t hi = std::max<uint32_t>(1, N >> kLoBits);
-        Fr* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, (size_t)(lo + hi) * sizeof(Fr));
+        void* mem = nullptr;
+        cudaError_t e = ctx->alloc(&mem, (size_t)(lo + hi) * sizeof(Fr));
         if (e != cudaSuccess) {
+            cudaGetLastError();
             delete d;
             set_error(std::string("domain tables: ") + cudaGetErrorString(e));
             return ERR_OOM;
         }
+        Fr* p = static_cast<Fr*>(mem);
         d->tables[r] = p;
         d->lo[r] = p;
         d->hi[r] = p + lo;
@@ -464,9 +467,10 @@ Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
             }
         }
     }
-    Fr* tw_mem = nullptr;
-    if (tw_elements && cudaMalloc(&tw_mem, tw_elements * sizeof(Fr)) == cudaSuccess) {
-        d->pass_tw_mem.push_back(tw_mem);
+    void* tw_all = nullptr;
+    if (tw_elements && ctx->alloc(&tw_all, tw_elements * sizeof(Fr)) == cudaSuccess) {
+        Fr* tw_mem = static_cast<Fr*>(tw_all);
+        d->pass_tw_mem.push_back(tw_all);
         for (const Table& t : tw) {
             k_pass_twiddles<<<grid_for(ctx, 1u << t.log_s, 256), 256, 0, ctx->stream>>>(
                 d->lo[t.root], d->hi[t.root], t.log_n, t.log_s, t.log_r, tw_mem);
@@ -478,7 +482,7 @@ Status domain_create(Context* ctx, uint32_t j, uint32_t k, Domain** out) {
         cudaGetLastError();
     }
     {
-        cudaError_t e = cudaMalloc(&d->d_tinv, (size_t)tlen * sizeof(Fr));
+        cudaError_t e = ctx->alloc(&d->d_tinv, (size_t)tlen * sizeof(Fr));
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d->d_tinv, d->t_inv.data(), (size_t)tlen * 32, cudaMemcpyHostToDevice, ctx->stream);
         // every table is ready for any stream from here on

@@ -918,7 +918,7 @@ Status keygen(Context* ctx, const Domain* d, const mzk_circuit_desc* cs, const m
     const size_t fr_elems = (size_t)F * (2 * n + E) + (size_t)P * (2 * n + E) + 3 * (size_t)E + (need_ones ? n : 0) +
                             uniq_total;
     const size_t bytes = fr_elems * sizeof(Fr) + (size_t)u * 4 * L + 256;
-    cudaError_t e = cudaMalloc(&key->mem, bytes);
+    cudaError_t e = ctx->alloc(&key->mem, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         set_error("keygen: device allocation of " + std::to_string(bytes) + " bytes failed");

@@ -104,7 +104,10 @@ struct Context {
     // device buffer `name` of at least `bytes` bytes (contents undefined)
     Status ensure(const char* name, size_t bytes, void** out);
     Status ensure_pinned(size_t bytes, void** out);
-    // the pair sums' buffer, of at least `bytes` bytes; null where it cannot be had
+    // cudaMalloc that takes the pair sums' buffer back before it fails
+    cudaError_t alloc(void** out, size_t bytes);
+    // the pair sums' buffer, of at least `bytes` bytes; null where it cannot be
+    // had.  Valid until the next ensure() that grows a buffer, alloc() or release.
     void* pair_memory(size_t bytes);
     void pair_release();
     ~Context();

@@ -77,3 +77,24 @@ def test_the_limit_frees_what_is_held(ctx):
     free0 = torch.cuda.mem_get_info(0)[0]
     ctx.set_msm_pair_memory(0)
     assert torch.cuda.mem_get_info(0)[0] - free0 >= scratch_bytes()
+
+
+def test_little_free_memory(ctx):
+    """What is needed gets the pair sums' memory back, and they take no more than a quarter of what is free."""
+    n = 1 << 20
+    ds, db = ctx.gen_rand_fr(59, n), ctx.gen_bases(61, n)
+    ctx.set_msm_window(13)
+    want = ctx.msm_device(ds, db, n)
+    rounds, _ = ctx.msm_last_pair_sums()
+    assert rounds > 0  # 1.9 GiB held: 10.5 and 5.3 M sums and the kernel's scratch
+    most = ctx.alloc(torch.cuda.mem_get_info(0)[0] - GIB)
+    need = ctx.alloc(2 * GIB)  # more than the 1 GiB left
+    assert np.array_equal(ctx.msm_device(ds, db, n), want)
+    assert ctx.msm_last_pair_sums() == (0, 0)
+    need.free()
+    assert torch.cuda.mem_get_info(0)[0] >= 2 * GIB  # enough for the sums, which leave it alone
+    assert np.array_equal(ctx.msm_device(ds, db, n), want)
+    assert ctx.msm_last_pair_sums() == (0, 0)
+    most.free()
+    assert np.array_equal(ctx.msm_device(ds, db, n), want)
+    assert ctx.msm_last_pair_sums()[0] == rounds
