@@ -719,9 +719,11 @@ int mzk_srs_read_processed(mzk_ctx *ctx, const uint8_t *bytes, size_t len, size_
  * request queue of create_proof requests (mzk_proof_request, any keys).  An
  * idle lane takes a wave: queued requests oldest first whose keys share the
  * first one's SRS buffer, while the wave holds fewer than max_batch proofs,
- * its device scratch stays within mem_budget_bytes / lanes and that of all
- * proofs in flight within mem_budget_bytes (0: no limit; a proof larger than
- * that runs alone when nothing else is in flight), run as one
+ * its device scratch (the proofs' polynomials and sorted MSM entries) stays
+ * within mem_budget_bytes / lanes and that of all proofs in flight within
+ * mem_budget_bytes (0: no limit; a proof larger than that runs alone when
+ * nothing else is in flight), less the quarter of it, at most 3.125 GiB a lane,
+ * that the MSMs' pair sums may hold; the wave is run as one
  * mzk_create_proofs call with `flags`; requests arriving while a wave runs
  * start beside it on the device.  max_batch = 1 with one lane and
  * MZK_PROVE_MSM_PER_CALL is the plain one-call-at-a-time prover.  A

@@ -15,6 +15,7 @@
 // With max_batch = 1 and one lane the same service is the plain
 // one-proof-at-a-time prover.  Latency is measured from submit to the moment
 // the wave that holds the request has its transcript on the host.
+#include <algorithm>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -60,6 +61,10 @@ struct Server {
     uint32_t max_batch = 1;
     uint32_t flags = 0;       // MZK_PROVE_* flags of every wave
     uint64_t mem_budget = 0;  // 0: no limit
+    // Of a lane's share, what its context may hold for the pair sums of its
+    // MSMs: up to a quarter (they halve the additions of large MSMs, while the
+    // rest holds the proofs of a wave).  Not available to admissions.
+    uint64_t pair_share = 0;
     uint64_t max_wave_rows = 0;  // 0: no limit on the rows (sum of 2^k) of one wave
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
@@ -80,7 +85,8 @@ struct Server {
         uint64_t rows = 0;
         // one wave takes at most its lane's share of the budget, so the other
         // lanes can admit requests beside it
-        const uint64_t lane_cap = mem_budget / lanes.size();
+        const uint64_t lane_cap = mem_budget / lanes.size() - pair_share;
+        const uint64_t all_cap = mem_budget - pair_share * lanes.size();
         const void* srs = queue.empty() ? nullptr : reqs[queue.front()]->srs;
         for (auto it = queue.begin(); it != queue.end() && batch.size() < max_batch;) {
             const Request& r = *reqs[*it];
@@ -95,7 +101,7 @@ struct Server {
             // the first proof of a wave is admitted when nothing else is in flight,
             // so a proof larger than the budget still runs (alone)
             const bool fits = mem_budget == 0 ||
-                              (in_flight_bytes + wave_after <= mem_budget && wave_after <= lane_cap) ||
+                              (in_flight_bytes + wave_after <= all_cap && wave_after <= lane_cap) ||
                               (in_flight_bytes == 0 && batch.empty());
             if (!fits) break;
             *bytes += r.bytes;
@@ -182,6 +188,8 @@ extern "C" int mzk_server_create(mzk_ctx* ctx, uint32_t max_batch, uint32_t lane
     s->impl.max_batch = max_batch;
     s->impl.mem_budget = mem_budget_bytes;
     s->impl.flags = flags;
+    if (mem_budget_bytes)
+        s->impl.pair_share = std::min<uint64_t>(mem_budget_bytes / lanes / 4, mzk::Context::kPairLimit);
     const int device = mzk::context_of(ctx)->device;
     for (uint32_t i = 0; i < lanes; i++) {
         mzk_ctx* lane = nullptr;
@@ -190,6 +198,7 @@ extern "C" int mzk_server_create(mzk_ctx* ctx, uint32_t max_batch, uint32_t lane
             delete s;
             return st;
         }
+        if (mem_budget_bytes) mzk::context_of(lane)->pair_limit = s->impl.pair_share;
         s->impl.lanes.push_back(lane);
     }
     for (mzk_ctx* lane : s->impl.lanes) s->impl.workers.emplace_back([s, lane] { s->impl.run(lane); });
