@@ -478,13 +478,13 @@ static __device__ __noinline__ PairCase pair_case(const Affine a, const Affine b
         c.kind = kPairFirst;
     } else if (!fp_is_zero(c.den)) {
         c.kind = kPairAdd;
-    } else if (!fp_is_zero(c.num)) {
+    } else if (!fp_is_zero(c.num) || fp_is_zero(a.y)) {  // b = -a
         c.kind = kPairInfinity;
     } else {
         const Fp xx = fp_mul(a.x, a.x);
         c.kind = kPairDouble;
         c.num = fp_add(fp_dbl(xx), xx);
-        c.den = fp_dbl(a.y);  // not zero: the curve has no point of order 2
+        c.den = fp_dbl(a.y);  // not zero: a zero here would spoil the sums of the whole batch
     }
     return c;
 }
