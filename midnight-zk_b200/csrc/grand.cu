@@ -316,7 +316,7 @@ cudaError_t launch_rec(const RecTasks& t, uint64_t n, uint64_t blocks, uint32_t 
 }
 
 // y[j] (n) from c[j] (n) with factor k[j]; in and out may not alias.
-// first_only: y[j] receives its first value alone (y[j][0]).
+// first_only (one task): y[0] receives its first value alone (y[0][0]).
 Status linrec_suffix_batch(Context* ctx, const Fr* const* c, Fr* const* y, const host::Fr4* k, uint32_t T, uint64_t n,
                            cudaStream_t st, bool first_only = false, int depth = 0) {
     if (n == 0 || T == 0) return OK;
@@ -362,16 +362,9 @@ Status linrec_suffix_batch(Context* ctx, const Fr* const* c, Fr* const* y, const
             }
             MZK_TRY(linrec_suffix_batch(ctx, sc.data(), sy.data(), kblock.data(), tb, blocks, st, first_only, depth + 1));
             if (first_only) continue;
-        } else if (first_only) {
-            // one block: its start is the first value
-            for (uint32_t j = 0; j < tb; j++) {
-                RecTasks one = t;
-                one.c[0] = t.c[j];
-                one.k[0] = t.k[j];
-                for (uint32_t l = 0; l < kRecLevels; l++) one.kk[0][l] = t.kk[j][l];
-                MZK_CUDA_CHECK(launch(one, 1, t.y[j], nullptr));
-                ctx->launches++;
-            }
+        } else if (first_only) {  // its start is the first value
+            MZK_CUDA_CHECK(launch(t, 1, t.y[0], nullptr));
+            ctx->launches++;
             continue;
         }
         MZK_CUDA_CHECK(launch(t, tb, nullptr, starts ? starts + blocks : nullptr));
