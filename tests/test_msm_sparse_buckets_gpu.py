@@ -70,3 +70,22 @@ def test_few_buckets_cost_no_more(ctx):
         return min(times)
 
     assert best(one) < 1.5 * best(uniform)
+
+
+def test_empty_buckets_are_cheap_to_reduce(ctx):
+    """2^22 scalars of 8 bits fill 255 of 1.9 M buckets; reducing them took as long as reducing full ones."""
+    n = 1 << 22
+    uniform, db, small = ctx.gen_rand_fr(109, n), ctx.gen_bases(113, n), ctx.alloc(n * 32)
+    values = np.stack([O.fr_op("from_canonical", np.array([v, 0, 0, 0], np.uint64)) for v in range(256)])
+    small.upload(values[np.random.default_rng(5).integers(0, 256, n)])
+
+    def reduce_ms(ds):
+        ctx.msm_device(ds, db, n)
+        ctx.set_profiling(True)
+        for _ in range(3):
+            ctx.msm_device(ds, db, n)
+        ms, calls = ctx.phase_stats()["reduce"]
+        ctx.set_profiling(False)
+        return ms / calls
+
+    assert reduce_ms(small) < 0.5 * reduce_ms(uniform)
