@@ -252,12 +252,13 @@ __device__ __forceinline__ Fr rec_chain(const Fr* __restrict__ c, uint64_t lo, u
     return acc;
 }
 
-// v <- sum_{u >= t} k^(K (u - t)) v_u over the block's threads (sm: kThreads)
-__device__ __forceinline__ Fr rec_scan(Fr v, const Fr* __restrict__ kk, Fr* sm) {
+// v <- sum_{u >= t} k^(K (u - t)) v_u over the block's threads (sm: kThreads);
+// live: threads from there on hold zero
+__device__ __forceinline__ Fr rec_scan(Fr v, const Fr* __restrict__ kk, Fr* sm, uint32_t live) {
     sm[threadIdx.x] = v;
     __syncthreads();
 #pragma unroll 1
-    for (uint32_t l = 0; l < kRecLevels; l++) {
+    for (uint32_t l = 0; l < kRecLevels && (1u << l) < live; l++) {
         const uint32_t off = 1u << l;
         const bool on = threadIdx.x + off < (uint32_t)kThreads;
         if (on) v = fr_add(v, fr_mul(kk[l], sm[threadIdx.x + off]));
@@ -268,6 +269,13 @@ __device__ __forceinline__ Fr rec_scan(Fr v, const Fr* __restrict__ kk, Fr* sm) 
     return v;
 }
 
+// threads of the block with elements below n, all of them where a carry comes in
+template <uint32_t K>
+__device__ __forceinline__ uint32_t rec_live(uint64_t n) {
+    const uint64_t first = (uint64_t)blockIdx.x * kThreads * K;
+    return (uint32_t)min((uint64_t)kThreads, (n - first + K - 1) / K);
+}
+
 // starts[task * stride + block] = the block's y at its first element with a zero carry-in
 template <uint32_t K>
 __global__ void __launch_bounds__(kThreads) k_rec_totals(const RecTasks t, uint64_t n, Fr* __restrict__ starts,
@@ -275,7 +283,7 @@ __global__ void __launch_bounds__(kThreads) k_rec_totals(const RecTasks t, uint6
     __shared__ Fr sm[kThreads];
     const uint32_t j = blockIdx.y;
     const uint64_t lo = ((uint64_t)blockIdx.x * kThreads + threadIdx.x) * K;
-    const Fr v = rec_scan(rec_chain<K>(t.c[j], lo, n, t.k[j]), t.kk[j], sm);
+    const Fr v = rec_scan(rec_chain<K>(t.c[j], lo, n, t.k[j]), t.kk[j], sm, rec_live<K>(n));
     if (threadIdx.x == 0) starts[j * stride + blockIdx.x] = v;
 }
 
@@ -295,7 +303,7 @@ __global__ void __launch_bounds__(kThreads) k_rec_solve(const RecTasks t, uint64
     if (has_carry) in = carry[j * stride + blockIdx.x + 1];
     // the carry enters as the value above the last thread's chunk
     if (has_carry && threadIdx.x == kThreads - 1) v = fr_add(v, fr_mul(t.kk[j][0], in));
-    rec_scan(v, t.kk[j], sm);
+    rec_scan(v, t.kk[j], sm, rec_live<K>(n));
     Fr acc = threadIdx.x + 1 < (uint32_t)kThreads ? sm[threadIdx.x + 1] : in;
 #pragma unroll
     for (int i = (int)K - 1; i >= 0; i--) {
