@@ -379,11 +379,13 @@ class DeviceBuffer:
         _check(lib().mzk_device_alloc(ctx.h, self.nbytes, ctypes.byref(p)))
         self.ptr = p.value
         ctx._buffers.add(self)
+        ctx._own("mzk_device_free", self.ptr)
 
     def free(self):
         if self.ptr and self.ctx.h:
-            _check(lib().mzk_device_free(self.ctx.h, self.ptr))
+            status = self.ctx._release("mzk_device_free", self.ptr)
             self.ptr = None
+            _check(status)
 
     def __del__(self):
         try:
@@ -439,6 +441,23 @@ class Context:
         # context goes
         self._servers, self._keys = weakref.WeakSet(), weakref.WeakSet()
         self._domains, self._buffers = weakref.WeakSet(), weakref.WeakSet()
+        # and their handles: collected in one cycle with its objects (at exit,
+        # say) the context may be finalised first, its weak references gone
+        self._handles = {destroy: set() for destroy in self.DESTROY}
+
+    # in the order in which they go
+    DESTROY = ("mzk_server_destroy", "mzk_plonk_key_destroy", "mzk_domain_destroy", "mzk_device_free")
+
+    def _own(self, destroy, handle):
+        self._handles[destroy].add(handle)
+
+    def _release(self, destroy, handle):
+        """Destroy a handle, unless this context is gone, which took it along."""
+        if handle not in self._handles[destroy]:
+            return 0
+        self._handles[destroy].discard(handle)
+        call = getattr(lib(), destroy)
+        return call(self.h, handle) if destroy == "mzk_device_free" else call(handle)
 
     def close(self):
         if getattr(self, "h", None):
@@ -450,6 +469,9 @@ class Context:
                     buf.free()
                 except MzkError:
                     pass
+            for destroy in self.DESTROY:
+                for handle in list(self._handles[destroy]):
+                    self._release(destroy, handle)
             lib().mzk_ctx_destroy(self.h)
             self.h = None
 
@@ -719,6 +741,7 @@ class EvaluationDomain:
         _check(lib().mzk_domain_create(ctx.h, j, k, ctypes.byref(h)))
         self.h = h.value
         ctx._domains.add(self)
+        ctx._own("mzk_domain_destroy", self.h)
         kk, ek = _u32(), _u32()
         _check(lib().mzk_domain_shape(self.h, ctypes.byref(kk), ctypes.byref(ek)))
         self.k, self.extended_k = kk.value, ek.value
@@ -727,7 +750,7 @@ class EvaluationDomain:
 
     def close(self):
         if getattr(self, "h", None):
-            lib().mzk_domain_destroy(self.h)
+            self.ctx._release("mzk_domain_destroy", self.h)
             self.h = None
 
     def __del__(self):
@@ -882,6 +905,7 @@ class ProvingServer:
         if max_wave_rows:
             _check(lib().mzk_server_set_wave_rows(self.h, int(max_wave_rows)))
         ctx._servers.add(self)
+        ctx._own("mzk_server_destroy", self.h)
         self._held = {}
 
     def submit(self, key, advice, blinds, instance=None):
@@ -910,7 +934,7 @@ class ProvingServer:
 
     def close(self):
         if getattr(self, "h", None):
-            lib().mzk_server_destroy(self.h)
+            self.ctx._release("mzk_server_destroy", self.h)
             self.h = None
 
     def __del__(self):
@@ -1193,6 +1217,7 @@ class PlonkKey:
         pc = circuit["perm_cols"]
         self.h = h.value
         ctx._keys.add(self)
+        ctx._own("mzk_plonk_key_destroy", self.h)
         repr_, plen, nbl = np.zeros(4, np.uint64), _sz(), _sz()
         _check(lib().mzk_plonk_key_info(self.h, _ptr(repr_), ctypes.byref(plen), ctypes.byref(nbl)))
         self.repr, self.proof_len, self.n_blinds = repr_, plen.value, nbl.value
@@ -1226,7 +1251,7 @@ class PlonkKey:
 
     def close(self):
         if getattr(self, "h", None):
-            lib().mzk_plonk_key_destroy(self.h)
+            self.ctx._release("mzk_plonk_key_destroy", self.h)
             self.h = None
 
     def __del__(self):
