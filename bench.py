@@ -41,9 +41,6 @@ sys.path.insert(0, str(ROOT))
 METRIC = "G1 MSM Mpts/s at 2^24"
 UNIT = "Mpts/s"
 IMAD_PER_FP_MUL = 600        # CIOS, 12 limbs: 2*12^2+12 = 300 products x (lo, hi)
-# per bucket entry at 2^24: three rounds of affine pair sums (7/8 of the entries, 5M + 1S
-# each, inversions left out), mixed additions (1/8, 8M + 2S)
-FP_MUL_PER_ENTRY = 6.5
 IMAD_PER_POINT_REF = 97.0e3  # reference schedule c=17, W=16 at 2^24: 1.628e12 IMAD / 2^24
 
 
@@ -131,8 +128,17 @@ class ClockSampler:
                 "power_w_max": max(r["power"] for r in rows), "samples": len(rows), "reasons": reasons}
 
 
-def traffic_from_profiles(c):
-    """DRAM bytes per bucket entry of the accumulation's kernels from the committed ncu summary."""
+def fp_mul_per_entry(rounds):
+    """Products per bucket entry: a round of affine pair sums (5M + 1S, inversions left out) halves the points that
+    are left, mixed additions (8M + 2S) take the rest."""
+    return sum(6 / 2 ** r for r in range(1, rounds + 1)) + 10 / 2 ** rounds
+
+
+def traffic_from_profiles(rounds):
+    """DRAM bytes per bucket entry of the accumulation's kernels from the committed ncu summary, whose capture has
+    three rounds of pair sums."""
+    if rounds != 3:
+        return None
     f = ROOT / "profiles" / "msm_accumulate.md"
     if not f.exists():
         return None
@@ -765,13 +771,14 @@ def run_ours(args):
     phases = ctx.phase_stats()
     ctx.set_profiling(False)
     c, windows, entries = ctx.msm_last_shape()
+    rounds, _ = ctx.msm_last_pair_sums()
     value = world * n / (ms / 1e3) / 1e6
 
     acc_ms, acc_cnt = phases["accumulate"]
     acc_avg_ms = acc_ms / max(acc_cnt, 1)
-    imad_acc = entries * FP_MUL_PER_ENTRY * IMAD_PER_FP_MUL
+    imad_acc = entries * fp_mul_per_entry(rounds) * IMAD_PER_FP_MUL
     achieved = imad_acc / (acc_avg_ms / 1e3)
-    tpe = traffic_from_profiles(c)
+    tpe = traffic_from_profiles(rounds)
     roofline = {
         "kernel": "k_pair_sums and k_accumulate (bucket accumulation)", "bound": "imad",
         "achieved": round(achieved / 1e12, 3), "peak": round(imad_peak / 1e12, 3), "unit": "TIMAD/s",
@@ -779,7 +786,7 @@ def run_ours(args):
         "traffic": None if tpe is None else round(tpe * entries),
         "peak_source": "measured in this run: max of mzk_probe_imad_peak's IMAD microbenchmarks and "
                        "600 x the measured 12-limb Montgomery multiplication rate (per-thread operands)",
-        "work": f"{entries} bucket entries x {FP_MUL_PER_ENTRY} Fp mul x {IMAD_PER_FP_MUL} IMAD",
+        "work": f"{entries} bucket entries x {fp_mul_per_entry(rounds)} Fp mul x {IMAD_PER_FP_MUL} IMAD",
         "launch_ms": round(acc_avg_ms, 3),
     }
     msm_roof = {

@@ -525,11 +525,13 @@ int mzk_msm_g1_device(mzk_ctx* ctx, const uint64_t* d_scalars, const uint64_t* d
 constexpr size_t kPipelineMinPoints = size_t(1) << 20;
 // Cumulative point fractions of the parts of a pipelined host MSM.  At 2^24
 // the upload (128 bytes a point at the host link's ~55 GB/s) takes ~39 ms
-// and the sort and accumulation ~84 ms, both linear in the points; every
+// and the sort and accumulation ~75 ms, both linear in the points; every
 // part after the first adds one bucket set that the reduction merges key by
 // key (one full XYZZ addition per key, ~4 ms at c = 20).  Three parts
 // balance the two: the compute stream waits for the first 12 % only, and
-// each later part is up before the one before it has been accumulated.
+// each later part is up before the one before it has been accumulated.  (The
+// fractions were chosen when every part was accumulated at the same rate, ~84 ms
+// in all; the first part has too few entries per bucket for pair sums.)
 constexpr int kHostParts = 3;
 constexpr double kPartEnd[kHostParts] = {0.12, 0.40, 1.0};
 static_assert(kHostParts <= mzk::kMaxMsmParts, "parts of a pipelined MSM");

@@ -2,7 +2,8 @@
 //
 // The algorithm of Bernstein and Yang, "Fast constant-time gcd computation and
 // modular inversion" (TCHES 2019/3), with the division step that starts at
-// delta = 1/2: from f = m, g = a, each step replaces (delta, f, g) by
+// delta = 1/2 (Pieter Wuille's variant, described with 30-bit limbs in
+// libsecp256k1's "The safegcd implementation in libsecp256k1 explained"): from f = m, g = a, each step replaces (delta, f, g) by
 // (1 - delta, g, (g - f)/2) if delta > 0 and g is odd, and by
 // (1 + delta, f, (g + (g mod 2) f)/2) otherwise, until g = 0 and f = +-1.
 // Thirty steps at a time depend on the low words of f and g only; they give a

@@ -18,19 +18,22 @@
 //                 random 4-byte writes leave L2 as whole sectors.  Zero digits
 //                 produce no entry, so zero and sparse scalars cost nothing
 //                 (msm_specific drops zero scalars).
-//  4. accumulate  the sorted entries split into equal chunks, one per thread:
+//  4. pair sums   for large inputs, up to three rounds that replace the points of
+//                 every bucket by the affine sums of neighbours, hundreds of
+//                 sums to one inversion (k_pair_sums).
+//  5. accumulate  the entries that are left split into equal chunks, one per thread:
 //                 every thread walks its chunk adding points into an XYZZ
 //                 accumulator (mixed addition, affine bases gathered from HBM).
 //                 Buckets entirely inside a chunk are written directly; a bucket
 //                 cut by a chunk edge leaves partial sums.  Equal chunks keep
 //                 every thread busy whatever the scalar distribution.
-//  5. fixup       the chunk where a cut bucket starts sums its partials.
-//  6. reduce      per window, sum_b (b+1) B_b by a tree over its buckets whose
+//  6. fixup       the chunk where a cut bucket starts sums its partials.
+//  7. reduce      per window, sum_b (b+1) B_b by a tree over its buckets whose
 //                 nodes carry their sum and the sums over every bit plane of
 //                 the index, four lanes per addition; where buckets fill the
 //                 GPU, running sums over groups of buckets come first.
-//  7. finish      one block per window shifts the planes and adds them up.
-//  8. host        sum_w 2^(c w) S_w (c doublings between windows) and the
+//  8. finish      one block per window shifts the planes and adds them up.
+//  9. host        sum_w 2^(c w) S_w (c doublings between windows) and the
 //                 affine normalisation on the host: a few hundred group
 //                 operations that one GPU thread would take ~1 ms for.
 #include <cuda_runtime.h>
@@ -360,9 +363,6 @@ __device__ __forceinline__ void chunk_range(uint32_t total, uint32_t t, uint32_t
     e = min(total, s + len);
 }
 
-// One flat loop over the chunk, so every thread of a warp runs the same number
-// of additions whatever its bucket boundaries; a boundary only costs a short
-// divergent flush.
 // The chunks that a cut bucket starts in, queued for k_fixup
 struct Owners {
     uint32_t* count;
@@ -381,8 +381,10 @@ __device__ __forceinline__ void flush_bucket(const Xyzz& acc, uint32_t k, uint32
     }
 }
 
-// kGather: entry j is the point sorted[j] (index | sign); otherwise point j of
-// `bases` itself (the pair sums of k_pair_sums).
+// One flat loop over the chunk, so every thread of a warp runs the same number
+// of additions whatever its bucket boundaries; a boundary only costs a short
+// divergent flush.  kGather: entry j is the point sorted[j] (index | sign);
+// otherwise point j of `bases` itself (the pair sums of k_pair_sums).
 template <bool kGather>
 __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __restrict__ bases,
                                                             const uint32_t* __restrict__ sorted,
@@ -450,9 +452,9 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumulate(const Affine* __r
 // products).  With ~40 products' worth of time for the inversion
 // (inv_divsteps) an addition costs ~7 products against the 10 of a mixed XYZZ
 // addition, at the price of writing the sums (96 bytes each) and reading them
-// again.  The multiply pipe is ~70 % busy (88 % in k_accumulate): the rest are
-// waits for loads that one sum's lead does not cover, instruction fetch and, with
-// two warps per scheduler, the latency of the products themselves.  A third
+// again.  The multiply pipe is ~75 % busy (88 % in k_accumulate): the rest are
+// waits for loads that one sum's lead does not cover and, with two warps per
+// scheduler, the latency of the products themselves.  A third
 // warp spills (168 registers) and is slower; the x coordinates two sums ahead
 // are 1 % slower.  Per call with 64 / 96 / 128 / 256 sums per inversion: 1000003
 // points 6.61 / 6.62 / 6.32 / 6.17 ms, 2^24 points 87.1 / 85.7 / 84.0 / 82.0, eight
@@ -894,9 +896,9 @@ __global__ void __launch_bounds__(kLongThreads) k_fixup_long(const Xyzz* __restr
 // whole tree takes ~2 nb additions, as many as running sums, and is only m
 // additions deep.  Then S = R + sum_t 2^t P_t.
 //
-// k_tree runs 1..8 heights of it per launch, each block a subtree in shared
-// memory with one quad of lanes per addition (a quad addition takes a third of
-// the time of a one-lane addition, and these are chains).  Where a call has
+// k_tree runs up to kTreeFirst heights of it per launch, each block a subtree in
+// shared memory with one quad of lanes per addition (a quad addition takes a third
+// of the time of a one-lane addition, and these are chains).  Where a call has
 // buckets enough to fill the GPU with one-lane work anyway (kTreeKeys),
 // k_group_sums first folds groups of L = 2^glen buckets by running sums
 // (R_g = sum of the group's buckets, T_g = sum_i (i+1) B_{gL+i}, ~1/4 less
@@ -908,7 +910,7 @@ __global__ void __launch_bounds__(kLongThreads) k_fixup_long(const Xyzz* __restr
 // multiply pipe for many.  Device time of the whole reduction, against running
 // sums over groups with one lane per addition, plane sums and a serial Horner
 // step per window: 4096 buckets (1000 points) 496 -> 94 us, 81920 (2^16
-// points) 1177 -> 265 us, 524288 (10^6 points) 1840 -> 1010 us.
+// points) 1177 -> 265 us, 524288 (10^6 points) 1846 -> 895 us.
 struct GroupWin {
     uint32_t key_start;    // first bucket key of the window
     uint32_t group_start;  // first running-sum group of the window
@@ -962,6 +964,7 @@ struct TreeWin {
     uint32_t v, b;
 };
 constexpr uint32_t kTreePoints = 256;  // points of a block's subtree (48 KB of shared memory)
+constexpr uint32_t kTreeFirst = 7;      // heights of a launch over single buckets, the most of any launch (plan_reduce)
 
 // Values are merged in place.  Value j of the node over the leaves from L sits
 // in slot (L, j), its new plane t in the last slot of leaf L + 2^t (the R that
@@ -1113,7 +1116,7 @@ ReducePlan plan_reduce(const std::vector<Window>& wins, uint32_t glen_log) {
             // 8.29 ms per call, 7 with 32 / 64 7.42 / 7.79, 8 with 32 / 64
             // 7.40 / 7.59; 65536 points: all within 3 %.
             uint32_t b = 0;
-            while (b < s.log_nodes && (s.v << (b + 1)) <= kTreePoints && !(s.v == 1 && b == 7)) b++;
+            while (b < s.log_nodes && (s.v << (b + 1)) <= kTreePoints && !(s.v == 1 && b == kTreeFirst)) b++;
             TreeWin t{blocks, s.start, (uint32_t)p.arena, s.v, b};
             const uint32_t n = 1u << (s.log_nodes - b);
             most = std::max(most, s.v << (b - 1));
@@ -1267,20 +1270,20 @@ cudaError_t launch_fixup(const Accumulation& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Rounds of pair sums for `entries` entries over `keys` buckets.  A sum costs
-// less than a mixed addition only while a thread has ~48 to share an inversion
-// (the lanes' grid has 37888 threads), and a round halves buckets of four
-// points or more.  Per call without / with 1 / 2 / 3 rounds, 64 sums per
-// inversion: 1000003 points (16.8
-// M entries, 32 per bucket) 7.34 / 6.86 / 6.73 / 6.66 ms, 4000000 points 25.4 /
-// 23.5 / 22.6 / 22.2, 2^24 points 92.0 / 90.0 / 88.0 / 87.4; 262144 points (5 M
-// entries) 2.60 / 2.59 / 2.59 / 2.62.
-constexpr uint64_t kPairsPerRound = 48 * 37888;
+// Rounds of pair sums by `threads` threads for `entries` entries over `keys`
+// buckets.  A sum costs less than a mixed addition only while a thread has ~48 to
+// share an inversion, and a round halves buckets of four points or more.  Per
+// call without and with them: 200000 points (4.0 M entries, one round) 2.10 and
+// 2.00 ms, 262144 (5.0 M) 2.51 and 2.36, 524288 (8.4 M, two) 4.29 and 3.96,
+// 1000003 (16.0 M, three) 7.28 and 6.15, 2^24 (218 M) 91.8 and 81.9.  The line was
+// set with batches of 64 sums, where 5.0 M entries gained nothing (2.60 and 2.59;
+// 1000003 points with 1 / 2 / 3 rounds 6.86 / 6.73 / 6.66).
+constexpr uint64_t kPairsPerThread = 48;
 constexpr int kPairRounds = 3;
 
-int pair_rounds(uint64_t entries, uint64_t keys) {
+int pair_rounds(uint64_t entries, uint64_t keys, uint64_t threads) {
     int r = 0;
-    while (r < kPairRounds && (entries >> (r + 1)) >= kPairsPerRound && (entries >> r) >= 4 * keys) r++;
+    while (r < kPairRounds && (entries >> (r + 1)) >= kPairsPerThread * threads && (entries >> r) >= 4 * keys) r++;
     return r;
 }
 
@@ -1383,9 +1386,9 @@ std::vector<PairPart> join_parts(const std::vector<uint2>& points, int rounds, u
 // upper bound (no zero digits); where it calls for rounds the true number,
 // which decides, is read back through `total` (pinned), with the split points
 // where the call may not fit one part.
-Status plan_pairs(Context* ctx, const Accumulation& all, uint64_t entries, uint64_t room, uint32_t* total,
-                  int* rounds, std::vector<PairPart>* parts, cudaStream_t st) {
-    *rounds = all.quad_blocks ? 0 : pair_rounds(entries, all.keys);
+Status plan_pairs(Context* ctx, const Accumulation& all, uint64_t entries, uint64_t threads, uint64_t room,
+                  uint32_t* total, int* rounds, std::vector<PairPart>* parts, cudaStream_t st) {
+    *rounds = all.quad_blocks ? 0 : pair_rounds(entries, all.keys, threads);
     if (!*rounds || !room) return OK;
     std::vector<uint2> points;
     if (pair_layout(entries, all.keys, *rounds).bytes > room) {
@@ -1404,7 +1407,7 @@ Status plan_pairs(Context* ctx, const Accumulation& all, uint64_t entries, uint6
     MZK_CUDA_CHECK(cudaMemcpyAsync(total, all.offsets + all.keys, 4, cudaMemcpyDeviceToHost, st));
     MZK_CUDA_CHECK(cudaStreamSynchronize(st));
     points.push_back(make_uint2(all.keys, *total));
-    *rounds = pair_rounds(*total, all.keys);
+    *rounds = pair_rounds(*total, all.keys, threads);
     if (*rounds) *parts = join_parts(points, *rounds, room);
     return OK;
 }
@@ -1418,8 +1421,8 @@ Status accumulate(Context* ctx, const Accumulation& all, uint64_t entries, uint3
     const size_t threads = (size_t)blocks * kPairThreads, fixed = align256(pair_scratch_bytes(threads));
     int rounds = 0;
     std::vector<PairPart> parts;
-    MZK_TRY(plan_pairs(ctx, all, entries, ctx->pair_limit > fixed ? ctx->pair_limit - fixed : 0, total, &rounds,
-                       &parts, st));
+    MZK_TRY(plan_pairs(ctx, all, entries, threads, ctx->pair_limit > fixed ? ctx->pair_limit - fixed : 0, total,
+                       &rounds, &parts, st));
     size_t need = 0;
     for (const PairPart& p : parts)
         need = std::max(need, p.paired ? pair_layout(p.entries, p.k1 - p.k0, rounds).bytes
@@ -1477,6 +1480,8 @@ Status accumulate(Context* ctx, const Accumulation& all, uint64_t entries, uint3
 
 // Window width by a cost model: W = ceil(256/c) windows of n mixed additions
 // (10 Fp mul) plus 2 * 2^(c-1) full additions (14 Fp mul) for the bucket sums.
+// The weights are those of an accumulation without pair sums and of running
+// sums; the widths were not fitted to today's kernels.
 int msm_pick_window(size_t n) {
     double best = 1e300;
     int bc = 8;
@@ -1942,9 +1947,11 @@ constexpr size_t kNaBucketsOff = kNaSortedOff + align256(kNaMaxWindows * kNoAllo
 constexpr size_t kNaPartialsOff = kNaBucketsOff + align256(kNaKeys * sizeof(Xyzz));
 constexpr size_t kNaQueueOff = kNaPartialsOff + align256(kNaAccThreads * 2 * sizeof(Xyzz));
 constexpr size_t kNaArenaOff = kNaQueueOff + align256(queue_bytes(kNaAccThreads));
-// the reduction tree's values over the widest key count: a node of 64 buckets
-// leaves 7 values, and the one or two launches above it far fewer
-constexpr size_t kNaArenaPoints = kNaKeys / 64 * 7 + kNaMaxWindows * 32;
+// the reduction tree's values: a node of the first launch's 2^7 buckets (every
+// window has as many) leaves 8 values, and up to 16 of those nodes per window
+// leave one of at most 12
+constexpr size_t kNaArenaPoints = (kNaKeys >> kTreeFirst) * (kTreeFirst + 1) + kNaMaxWindows * 12;
+static_assert(kNoAllocMinC - 1 >= (int)kTreeFirst && kNoAllocMaxC - 1 <= (int)kTreeFirst + 4, "two launches of the tree");
 constexpr size_t kNaTabBytes = kNaMaxWindows * (4 * sizeof(TreeWin) + sizeof(FinWin));
 constexpr size_t kNaWsumOff = kNaArenaOff + align256(kNaArenaPoints * sizeof(Xyzz));
 constexpr size_t kNaScanOff = kNaWsumOff + align256(kNaMaxWindows * sizeof(Xyzz));
